@@ -24,6 +24,8 @@ int pick_impl(const float* part_max, const int32_t* part_idx, int partials, cons
               int64_t* tok, int32_t* pos, uint8_t* finished, const int64_t* forced, int max_prompt,
               const int32_t* plen, const int32_t* limit, int64_t* out, int out_cols, int eos, int64_t* argmax,
               uint8_t* flags_host, int pdl, void* stream);
+bool fused_step_applies(const b200dec_plan* pl, int row0, int rows);
+int fused_step(const b200dec_plan* pl, int rows, void* stream);
 }  // namespace b200dec_detail
 
 using namespace b200dec_detail;
@@ -56,6 +58,7 @@ int b200dec_sizeof(int which) {
 // not hold the rows goes in two passes) and two attention kernels, the vocabulary projection, the pick.
 int b200dec_step_launches(const b200dec_plan* pl, int rows) {
   if (!pl || !pl->layer || rows < 1) return 0;
+  if (fused_step_applies(pl, 0, rows)) return 1;
   const bool linked = pl->xh && pl->ln_stats && pl->a_kind == B200DEC_A_F16 && pl->layer[0].qkv.kind != B200DEC_W_BF16;
   const int ln_kind = linked ? B200DEC_A_F16_ROWS16 : pl->a_kind;
   int n = 2;  // embedding, pick
@@ -77,6 +80,7 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
   B200_REQUIRE(pl->heads * pl->head_dim == D_MODEL, "step: heads * head_dim must be %d", D_MODEL);
   B200_REQUIRE(pl->vocab == pl->head.n, "step: vocab %d vs head rows %d", pl->vocab, pl->head.n);
   B200_REQUIRE(!(pl->kv_int8 && pl->attn_ring), "step: the ring attention kernel reads bf16 caches only");
+  if (fused_step_applies(pl, row0, rows)) return fused_step(pl, rows, stream);  // up to 16 rows: one kernel (step_fused.cuh)
   const int hd = pl->heads * pl->head_dim;
   const int want = pl->classes ? pl->classes : 7;  // 1 embedding / vocabulary projection / pick, 2 projections, 4 attention
   // which launches carry the programmatic-dependent-launch attribute: bit 0 a projection (or the pick) that follows a

@@ -55,7 +55,8 @@ class Plan(C.Structure):
                 ("finished", vp), ("forced", vp), ("out", vp), ("flags_host", vp), ("status", vp),
                 ("x", vp), ("qkv", vp), ("cq", vp), ("att", vp), ("mid", vp),
                 ("attn_part", vp), ("attn_count", vp), ("head_max", vp), ("head_idx", vp),
-                ("xh", vp), ("ln_stats", vp), ("sched_self", vp), ("sched_cross", vp), ("logits", vp), ("argmax", vp)]
+                ("xh", vp), ("ln_stats", vp), ("sched_self", vp), ("sched_cross", vp), ("logits", vp), ("argmax", vp),
+                ("fused_ws", vp * 16)]
 
 
 # name -> (restype, argtypes); every symbol include/b200dec.h declares
@@ -120,6 +121,7 @@ PROTOTYPES = {
     "b200dec_admit_record_ints": (C.c_int, [C.c_int]),
     "b200dec_compact_active": (C.c_int, [C.POINTER(Plan), C.c_int, vp, vp, C.c_int, vp]),
     "b200dec_step": (C.c_int, [C.POINTER(Plan), C.c_int, vp]),
+    "b200dec_fused_words": (i64, [C.POINTER(Plan), C.c_int]),
     "b200dec_step_rows": (C.c_int, [C.POINTER(Plan), C.c_int, C.c_int, vp]),
     "b200dec_step_launches": (C.c_int, [C.POINTER(Plan), C.c_int]),
 }

@@ -19,6 +19,7 @@ the register-dequantising mma.sync kernel from a second packing of the same weig
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 import torch
@@ -31,6 +32,13 @@ ACTS = {"relu": nv.ACT_RELU, "gelu": nv.ACT_GELU}
 
 def _fp32(t: torch.Tensor) -> torch.Tensor:
     return t.detach().float().contiguous()
+
+
+def _image(n: int, device) -> torch.Tensor:
+    """n bytes on a 1 KB boundary (the swizzle atom of the tile images; the allocator gives 512)."""
+    buf = torch.empty(n + 1024, dtype=torch.uint8, device=device)
+    at = -buf.data_ptr() % 1024
+    return buf[at:at + n]
 
 
 class _Layer:
@@ -79,7 +87,7 @@ class _PrefillWeight:
         self.n, self.k = -(-n // 256) * 256, k
         wb = torch.zeros(self.n, k, dtype=torch.bfloat16, device=w.device)
         wb[:n] = w.detach().to(torch.bfloat16)
-        self.image = torch.empty(self.n * k * 2, dtype=torch.uint8, device=w.device)
+        self.image = _image(self.n * k * 2, w.device)
         nv.check(nv.lib().b200dec_prefill_tile_weight(nv.ptr(wb), self.n, k, nv.ptr(self.image), nv.stream_ptr()))
         torch.cuda.current_stream().synchronize()
         self.bias = torch.zeros(self.n, device=w.device)
@@ -95,7 +103,7 @@ class StreamDecoder:
                  head_split: bool = True, keep_reference: bool = False, chains: int = 1, attn_ring: bool = False,
                  head_umma: bool = True, kv_int8: bool = False, proj_umma: bool | str = True,
                  kv_prefetch_mb: int = 0, device_sched: bool = False, fp16_weights: bool = False,
-                 umma_above_rows: int = 16,
+                 umma_above_rows: int = 16, fused_rows: int = 16,
                  _packed: tuple | None = None):
         """model: a CohereAsrForConditionalGeneration-shaped module on a CUDA device (see synth.synthetic_model).
         int8: weight-only int8 with per-output-channel scales on every projection (fp16 activations, fp32
@@ -116,7 +124,8 @@ class StreamDecoder:
         appends to it, every step drops the rows that ended and leaves the live count in `live` (pinned), so a
         scheduler never calls set_active after an eviction. umma_above_rows: the tcgen05 layer projections serve the
         buckets of more than this many rows, the smaller buckets run a second, mma.sync packing of the same weights
-        (0: tcgen05 in every bucket)."""
+        (0: tcgen05 in every bucket). fused_rows: buckets of up to this many rows (at most 16) run a step as one
+        cooperative kernel where the mode allows it (csrc/step_fused.cuh; 0: as the sequence of kernels)."""
         nv.lib()  # fail now, loudly, if the CUDA library is missing
         assert not ffn_sparse or int8, "2:4 feed-forward weights are int8"
         assert not (fp16_weights and int8), "fp16_weights is a mode of its own beside int8"
@@ -233,6 +242,7 @@ class StreamDecoder:
             self.chains = max(1, int(chains))
             self.side_streams = [torch.cuda.Stream(device=dev, priority=-1) for _ in range(self.chains - 1)]
             self._build_plan()
+            self._fused_ws = self._fused_workspaces(fused_rows)
             self._select_layers(min(self.buckets))
             self.launches_per_step = lib.b200dec_step_launches(C.byref(self.plan), min(self.buckets))
             self.weight_bytes = sum(p.stream_bytes() for ly in self.layers for p in ly.projections()) + \
@@ -294,7 +304,8 @@ class StreamDecoder:
         self.head = packed("head")
         for name in ("proj", "cross"):
             w = object.__new__(_PrefillWeight)
-            w.image, w.bias = t[f"prefill.{name}.image"], t[f"prefill.{name}.bias"]
+            w.image, w.bias = _image(t[f"prefill.{name}.image"].numel(), self.device), t[f"prefill.{name}.bias"]
+            w.image.copy_(t[f"prefill.{name}.image"])
             w.n, w.k = manifest["prefill"][name]
             setattr(self, name, w)
 
@@ -398,6 +409,37 @@ class StreamDecoder:
         p.flags_host = self.flags.data_ptr()
         self.plan = p
 
+    def _fused_workspaces(self, fused_rows: int) -> dict[int, torch.Tensor]:
+        """Exchange buffers of the buckets whose step is one kernel, by rows (their initial state: reset())."""
+        ws = {}
+        if self.chains == 1 and not self.attn_ring:
+            for b in (b for b in self.buckets if b <= min(fused_rows, 16)):
+                self._select_layers(b)
+                words = nv.lib().b200dec_fused_words(C.byref(self.plan), b)
+                if words:
+                    ws[b] = torch.empty(words, device=self.device, dtype=torch.int32)
+                    self.plan.fused_ws[b - 1] = ws[b].data_ptr()
+        for t in ws.values():
+            t.fill_(-1)
+            t[0] = 0
+        torch.cuda.current_stream().synchronize()
+        return ws
+
+    # The CTAs of a fused step wait for one another, so two of them must not share the GPU: a decoder whose stream takes
+    # over from another decoder's waits for what that one has been given so far.
+    _fused_lock = threading.Lock()
+    _fused_stream: dict[int, torch.cuda.Stream] = {}
+
+    def _fused_turn(self) -> None:
+        """Call with the lock held, before a fused step is launched on the decoder stream."""
+        last = self._fused_stream.get(self.device.index)
+        if last is not self.stream:
+            if last is not None:
+                done = torch.cuda.Event()
+                done.record(last)
+                self.stream.wait_event(done)
+            self._fused_stream[self.device.index] = self.stream
+
     def _select_layers(self, b: int) -> None:
         """Points the plan at the layer packings bucket b runs on (a captured graph keeps what it was captured with)."""
         small = self._layer_structs_small is not None and b <= self._small_rows
@@ -454,7 +496,9 @@ class StreamDecoder:
         pool = torch.cuda.graph_pool_handle()
         with torch.cuda.device(self.device), torch.cuda.stream(self.stream):
             for rows in sorted(self.buckets, reverse=True):
-                self._step(rows)
+                with self._fused_lock:
+                    self._fused_turn()
+                    self._step(rows)
                 self.stream.synchronize()
                 graph = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(graph, pool=pool, stream=self.stream):
@@ -601,11 +645,19 @@ class StreamDecoder:
         """One decoding step of `bucket` rows on the decoder stream (a graph replay)."""
         torch.cuda.nvtx.range_push("b200dec.step")
         with torch.cuda.stream(self.stream):
-            if self.use_graphs:
-                self.graphs[bucket].replay()
+            if bucket in self._fused_ws:
+                with self._fused_lock:
+                    self._fused_turn()
+                    self._launch_step(bucket)
             else:
-                self._step(bucket)
+                self._launch_step(bucket)
         torch.cuda.nvtx.range_pop()
+
+    def _launch_step(self, bucket: int) -> None:
+        if self.use_graphs:
+            self.graphs[bucket].replay()
+        else:
+            self._step(bucket)
 
     # ---- identity of the packed weights -----------------------------------------------------------------------------
 

@@ -143,6 +143,12 @@ typedef struct b200dec_plan {
   /* optional recording (tests, teacher forcing); NULL in production */
   float* logits;       /* (rows, vocab) */
   int64_t* argmax;     /* (slots + 1): the un-forced greedy choice of each slot's last step */
+  /* fused_ws[r - 1]: workspace of b200dec_fused_words(plan, r) words, 16-byte aligned, with which a step of r rows runs
+   * as ONE cooperative kernel (csrc/step_fused.cuh); NULL: as the sequence of kernels. Before its first use word 0 is 0 and
+   * every other word is 0xffffffff (again after a step that reported B200DEC_ST_TIMEOUT was cut short by its caller). The
+   * kernel's CTAs wait for one another, so the caller keeps fused steps of different streams from running at the same
+   * time on one device. withhold bit 2 (tests only): one CTA leaves out one result, so the waits for it run out. */
+  void* fused_ws[16];
 } b200dec_plan;
 
 const char* b200dec_last_error(void);
@@ -377,6 +383,10 @@ int b200dec_compact_active(const b200dec_plan* plan, int rows, int32_t* n_active
 /* The whole step for `rows` rows: embed, `layers` layers, head, pick. Replaces StreamDecoder._step
  * (kernels/stream_decoder.py:176-199); its D2H copy of the flags becomes plan->flags_host, or stays with the caller. */
 int b200dec_step(const b200dec_plan* plan, int rows, void* stream);
+/* 32-bit words of the workspace with which a step of `rows` rows runs as one kernel (plan->fused_ws[rows - 1]), or 0 when
+ * this plan's steps of that size do not: more than 16 rows, weight kinds other than the mma.sync packings, the ring
+ * attention kernel, a device of fewer than 128 SMs. */
+int64_t b200dec_fused_words(const b200dec_plan* plan, int rows);
 /* The same for rows [row0, row0 + rows) of the step's batch only. Disjoint row ranges share no scratch, so a caller
  * may run several ranges concurrently on forked streams to overlap one range's attention (bound by HBM) with another's
  * projections (bound by latency). No counterpart in the reference, which runs the batch as one chain. */

@@ -3,6 +3,7 @@ seeded weights and inputs. Tolerances are the ones the benchmark definition stat
 max-abs of the fp32 path on the weights the mode stores (dequantised int8 / bf16-rounded), greedy agreement >= 99.5 %
 under teacher forcing."""
 
+import functools
 import os
 
 import numpy as np
@@ -366,6 +367,62 @@ def test_bounded_wait_runs_out_and_the_context_survives(bit, what, slots, bucket
         dec.status.zero_()
     got, _ = _run_teacher_forced(dec, memory, prompts, 4)
     assert np.array_equal(got, want), what
+
+
+@functools.lru_cache(maxsize=2)
+def _two_layers(heads):
+    return synthetic_model(3, heads=heads, head_dim=1024 // heads, act="gelu" if heads == 16 else "relu", layers=2,
+                           bias_std=0.05)
+
+
+@pytest.mark.parametrize("heads", [16, 8])
+@pytest.mark.parametrize("mode", [dict(int8=True), dict(int8=True, ffn_sparse=True), dict(fp16_weights=True), dict()])
+@pytest.mark.parametrize("kv_int8", [False, True])
+@pytest.mark.parametrize("rows", [1, 8, 9, 16])
+def test_fused_step_gives_what_the_kernel_sequence_gives(heads, mode, kv_int8, rows):
+    """Up to 16 rows a step runs as one cooperative kernel: the logits of the first and of later steps, the tokens and
+    the positions are those of the kernel sequence. Row counts on both sides of the kernel's operand tiles (8, 16) and
+    of one (row, head) per CTA (128 of them); contexts from the empty cache and one frame to more keys than one round
+    of a warp's loads. Both sides stay within LOGIT_TOL of the oracle elsewhere; here they are held to it against one
+    another (fp16 operands, other summation orders)."""
+    model = _two_layers(heads)
+    rng = np.random.default_rng(rows)
+    frames = np.linspace(1, 300, rows).astype(int).tolist() if rows > 1 else [300]
+    memory = [rng.standard_normal((t, 1024)).astype(np.float32) for t in frames]
+    prompts = [rng.integers(0, 16384, 150).astype(np.int64) for _ in range(rows)]
+    got = []
+    for fused_rows in (0, 16):
+        dec = _decoder(model, slots=rows, buckets=(rows,), max_new_tokens=8, max_prompt=150, max_audio_s=30.0, eos=-1,
+                       record=True, kv_int8=kv_int8, fused_rows=fused_rows, **mode)
+        assert dec.launches(rows) == 1 if fused_rows else dec.launches(rows) > 1
+        lg, _ = _run_teacher_forced(dec, memory, prompts, 150)
+        got.append((lg[[0, 1, 2, 40, 149]], dec.out.cpu().numpy()[:, :150], dec.pos.cpu().numpy()))
+    assert np.abs(got[0][0] - got[1][0]).max() <= LOGIT_TOL
+    assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])
+
+
+def test_fused_step_bounded_wait_runs_out_and_the_context_survives():
+    """The fused step's waits for other CTAs' results: with a short limit and one CTA leaving a result out, they run
+    out, the kernel returns, the status word says so, and the next steps give the bits they gave before."""
+    from cohere_inference_b200 import native as nv
+    model = synthetic_model(0, layers=2)
+    rng = np.random.default_rng(5)
+    memory = [rng.standard_normal((60, 1024)).astype(np.float32) for _ in range(3)]
+    prompts = [rng.integers(0, 16384, 6).astype(np.int64) for _ in range(3)]
+    dec = _decoder(model, slots=4, max_new_tokens=8, max_prompt=8, max_audio_s=10.0, eos=-1, record=True, graphs=False,
+                   int8=True)
+    want, _ = _run_teacher_forced(dec, memory, prompts, 4)
+    dec.admit([0, 1, 2], [torch.from_numpy(p) for p in prompts], [60] * 3)
+    dec.plan.wait_limit, dec.plan.withhold = 2048, 4
+    assert dec.launches(4) == 1
+    dec.step(dec.set_active([0, 1, 2]))
+    with pytest.raises(nv.NativeError, match="bounded wait"):
+        dec.check_status()
+    dec.plan.wait_limit, dec.plan.withhold = 0, 0
+    with torch.cuda.stream(dec.stream):
+        dec.status.zero_()
+    got, _ = _run_teacher_forced(dec, memory, prompts, 4)
+    assert np.array_equal(got, want)
 
 
 def test_small_buckets_point_at_the_mma_sync_packing():
