@@ -4,13 +4,16 @@
 // (frames x 16384) intermediate and no library GEMM.
 //
 // One kernel computes C(M, N) = A(M, K) B(N, K)^T + bias with fp32 activations A and bf16 weights B:
-//   * A is split into two bf16 halves, A = Ah + Al (about 16 bits of mantissa), and the product is Ah B^T + Al B^T,
-//     i.e. one bf16 GEMM over K' = 2 K whose second half re-reads the same weights. Both operands are stored in global
-//     memory as the exact shared-memory image of their tiles (K-major rows of 128 bytes with the 128-byte swizzle,
-//     16 KB per 128-row block of A, 32 KB per 256-channel block of B), so a pipeline stage is two plain
-//     cp.async.bulk copies that complete on an mbarrier; nothing else touches the operands.
-//   * persistent CTAs, one per SM, walk the (n tile, m tile) list; warp 0 feeds a 4-stage ring, warp 1 issues
-//     tcgen05.mma (M 128, N 256, K 16; 4 per stage) into one of two 256-column accumulators in tensor memory and
+//   * A is split into two bf16 halves, A = Ah + Al (about 16 bits of mantissa), and the product is Ah B^T + Al B^T. Both
+//     operands are stored in global memory as the exact shared-memory image of their tiles (K-major rows of 128 bytes
+//     with the 128-byte swizzle, 16 KB per 128-row block of a half of A, 32 KB per 256-channel block of B), so a pipeline
+//     stage is three plain cp.async.bulk copies that complete on an mbarrier; nothing else touches the operands. A stage
+//     holds 64 k of both halves and of the weights, so that the weights enter shared memory once: the multiply of a
+//     stage takes 1024 cycles, its 64 KB at 64 bytes a cycle from L2 as long. (As one product over 2 K with the weights
+//     fetched for either half it was 96 KB, and bound by them: 64 clips, 13 600 frames, 906 -> 819 us a
+//     prefill, 1.04 -> 1.18 PFLOP/s of the two halves.)
+//   * persistent CTAs, one per SM, walk the (n tile, m tile) list; warp 0 feeds a 3-stage ring, warp 1 issues
+//     tcgen05.mma (M 128, N 256, K 16; 8 per stage) into one of two 256-column accumulators in tensor memory and
 //     commits stage releases and tile completion to mbarriers, warps 2-5 drain the other accumulator with tcgen05.ld
 //     (a thread owns one frame = one tensor-memory lane) while the next tile multiplies.
 //   * epilogues: (0) the result, split again into bf16 halves, in the operand image of the next product; (1) a head
@@ -25,8 +28,8 @@ using namespace b200dec_detail;
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
-constexpr int A_STAGE = BM * BK * 2, B_STAGE = BN * BK * 2, STAGE_BYTES = A_STAGE + B_STAGE;
+constexpr int BM = 128, BN = 256, BK = 64, STAGES = 3;
+constexpr int A_STAGE = BM * BK * 2, B_STAGE = BN * BK * 2, STAGE_BYTES = 2 * A_STAGE + B_STAGE;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // slack to align the base to a swizzle atom
 constexpr int NTHREADS = 192;                            // producer warp, MMA warp, four epilogue warps
 constexpr uint32_t WAIT_LIMIT = 1u << 20;
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
   __shared__ uint32_t tmem_base;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int MT = (p.M + BM - 1) / BM, NT = p.N / BN, NKB = p.K / BK, NKB2 = 2 * NKB;
+  const int MT = (p.M + BM - 1) / BM, NT = p.N / BN, NKB = p.K / BK;
   const int tiles = MT * NT;
 
   if (tid == 0) {
@@ -184,20 +187,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
   const uint32_t tmem_d = tmem_base;
 
   if (warp == 0) {
-    // ---- producer: two bulk copies per stage --------------------------------------------------------------------------
+    // ---- producer: three bulk copies per stage -------------------------------------------------------------------------
     if (lane == 0) {
       bool ok = true;
       uint32_t it = 0;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
         const int mt = tile % MT, nt = tile / MT;
-        for (int kb = 0; kb < NKB2; ++kb, ++it) {
+        for (int kb = 0; kb < NKB; ++kb, ++it) {
           const int s = it % STAGES;
           ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1);
           if (!ok) break;
           unsigned char* st = smem + s * STAGE_BYTES;
           mbar_expect_tx(&full[s], STAGE_BYTES);
-          bulk_load(st, p.a + ((size_t)mt * NKB2 + kb) * A_STAGE, A_STAGE, &full[s]);
-          bulk_load(st + A_STAGE, p.w + ((size_t)nt * NKB + kb % NKB) * B_STAGE, B_STAGE, &full[s]);
+          const unsigned char* a = p.a + ((size_t)mt * 2 * NKB + kb) * A_STAGE;
+          bulk_load(st, a, A_STAGE, &full[s]);
+          bulk_load(st + A_STAGE, a + (size_t)NKB * A_STAGE, A_STAGE, &full[s]);
+          bulk_load(st + 2 * A_STAGE, p.w + ((size_t)nt * NKB + kb) * B_STAGE, B_STAGE, &full[s]);
         }
       }
       if (!ok) {
@@ -221,14 +226,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
         if (!ok) break;
         tc_fence_after();
         const uint32_t acc = tmem_d + buf * BN;
-        for (int kb = 0; kb < NKB2; ++kb, ++it) {
+        for (int kb = 0; kb < NKB; ++kb, ++it) {
           const int s = it % STAGES;
           ok = mbar_wait(&full[s], (it / STAGES) & 1);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a0 = smem_u32(smem + s * STAGE_BYTES), b0 = a0 + A_STAGE;
+          const uint32_t a0 = smem_u32(smem + s * STAGE_BYTES), b0 = a0 + 2 * A_STAGE;
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_bf16(acc, umma_desc(a0 + k * 32), umma_desc(b0 + k * 32), (kb | k) != 0);
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k)
+              umma_bf16(acc, umma_desc(a0 + h * A_STAGE + k * 32), umma_desc(b0 + k * 32), (kb | h | k) != 0);
           umma_commit(&empty[s]);  // the stage is free once these MMAs have read it
         }
         if (ok) umma_commit(&tfull[buf]);
