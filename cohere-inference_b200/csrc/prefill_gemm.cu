@@ -11,7 +11,7 @@
 //     holds 64 k of both halves and of the weights, so that the weights enter shared memory once: the multiply of a
 //     stage takes 1024 cycles, its 64 KB at 64 bytes a cycle from L2 as long. (As one product over 2 K with the weights
 //     fetched for either half it was 96 KB, and bound by them: 64 clips, 13 600 frames, 906 -> 819 us a
-//     prefill, 1.04 -> 1.18 PFLOP/s of the two halves.)
+//     prefill, 1.07 -> 1.18 PFLOP/s of the two halves.)
 //   * persistent CTAs, one per SM, walk the (n tile, m tile) list; warp 0 feeds a 3-stage ring, warp 1 issues
 //     tcgen05.mma (M 128, N 256, K 16; 8 per stage) into one of two 256-column accumulators in tensor memory and
 //     commits stage releases and tile completion to mbarriers, warps 2-5 drain the other accumulator with tcgen05.ld
@@ -28,12 +28,21 @@ using namespace b200dec_detail;
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 3;
-constexpr int A_STAGE = BM * BK * 2, B_STAGE = BN * BK * 2, STAGE_BYTES = 2 * A_STAGE + B_STAGE;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // slack to align the base to a swizzle atom
+constexpr int BM = 128, BN = 256, BK = 64;
+constexpr int A_STAGE = BM * BK * 2, B_BLOCK = BN * BK * 2;
+// TN: channels of a CTA's tile. 256, or 64 (a quarter of a weight block: 64 rows of 128 bytes, contiguous) where that
+// still is one wave.
+template <int TN>
+struct Tile {
+  static constexpr int STAGES = TN == BN ? 3 : 5, B_STAGE = TN * BK * 2, STAGE_BYTES = 2 * A_STAGE + B_STAGE;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // slack to align the base to a swizzle atom
+  static constexpr int TMEM_COLS = 2 * TN;                        // two accumulators
+  // bf16 x bf16 -> fp32, both operands K-major, M = 128, N = TN
+  static constexpr uint32_t IDESC =
+      (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+};
 constexpr int NTHREADS = 192;                            // producer warp, MMA warp, four epilogue warps
 constexpr uint32_t WAIT_LIMIT = 1u << 20;
-constexpr int TMEM_COLS = 512;                           // two accumulators of 256 columns
 
 struct GemmArgs {
   const unsigned char* a;  // operand image of the rows: [m tile][2 K / 64][16 KB]
@@ -41,6 +50,7 @@ struct GemmArgs {
   const float* bias;       // (N) or null
   int M, N, K;
   int mode;                // 0 operand image of the next product, 1 bf16 caches, 2 int8 caches
+  int halves;              // of A: 2, or 1 when the rows are bf16 values (their low halves are zero, and not read)
   unsigned char* next;     // mode 0: [m tile][2 N / 64][16 KB]
   const int4* pieces;      // modes 1, 2: (n_pieces) {first row, frames, slot, 0}, first rows ascending from 0
   int n_pieces;
@@ -92,12 +102,10 @@ DEVI uint64_t umma_desc(uint32_t saddr) {
   d |= (uint64_t)2 << 61;
   return d;
 }
-// bf16 x bf16 -> fp32, both operands K-major, M = 128, N = 256
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-DEVI void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+DEVI void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(IDESC), "r"(accumulate)
+      "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 DEVI void umma_commit(uint64_t* bar) {
@@ -160,14 +168,16 @@ DEVI void store_q8_64(const float (&f)[64], float mx, int8_t* dst) {
   }
 }
 
+template <int TN>
 __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArgs p) {
+  constexpr int STAGES = Tile<TN>::STAGES, B_STAGE = Tile<TN>::B_STAGE, STAGE_BYTES = Tile<TN>::STAGE_BYTES;
   extern __shared__ unsigned char dyn_smem[];
   unsigned char* smem = dyn_smem + ((1024 - (smem_u32(dyn_smem) & 1023)) & 1023);
   __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2];
   __shared__ uint32_t tmem_base;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int MT = (p.M + BM - 1) / BM, NT = p.N / BN, NKB = p.K / BK;
+  const int MT = (p.M + BM - 1) / BM, NT = p.N / TN, NKB = p.K / BK;
   const int tiles = MT * NT;
 
   if (tid == 0) {
@@ -175,9 +185,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
     for (int i = 0; i < 2; ++i) mbar_init(&tfull[i], 1), mbar_init(&tempty[i], 4);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // The rows (and the caches, and the piece table) are those of the kernels before. Ahead of the allocation, so that no
+  // CTA sits on tensor memory while it waits.
+  pdl_wait();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "n"(TMEM_COLS)
+                 "n"(Tile<TN>::TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -185,6 +198,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_d = tmem_base;
+  pdl_trigger();
 
   if (warp == 0) {
     // ---- producer: three bulk copies per stage -------------------------------------------------------------------------
@@ -198,11 +212,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
           ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1);
           if (!ok) break;
           unsigned char* st = smem + s * STAGE_BYTES;
-          mbar_expect_tx(&full[s], STAGE_BYTES);
+          mbar_expect_tx(&full[s], p.halves * A_STAGE + B_STAGE);
           const unsigned char* a = p.a + ((size_t)mt * 2 * NKB + kb) * A_STAGE;
           bulk_load(st, a, A_STAGE, &full[s]);
-          bulk_load(st + A_STAGE, a + (size_t)NKB * A_STAGE, A_STAGE, &full[s]);
-          bulk_load(st + 2 * A_STAGE, p.w + ((size_t)nt * NKB + kb) * B_STAGE, B_STAGE, &full[s]);
+          if (p.halves > 1) bulk_load(st + A_STAGE, a + (size_t)NKB * A_STAGE, A_STAGE, &full[s]);
+          const int n0 = nt * TN;
+          bulk_load(st + 2 * A_STAGE, p.w + ((size_t)(n0 / BN) * NKB + kb) * B_BLOCK + n0 % BN / TN * B_STAGE, B_STAGE, &full[s]);
         }
       }
       if (!ok) {
@@ -225,18 +240,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
         ok = mbar_wait(&tempty[buf], ((tc >> 1) & 1) ^ 1);  // the epilogue has drained this accumulator
         if (!ok) break;
         tc_fence_after();
-        const uint32_t acc = tmem_d + buf * BN;
+        const uint32_t acc = tmem_d + buf * TN;
         for (int kb = 0; kb < NKB; ++kb, ++it) {
           const int s = it % STAGES;
           ok = mbar_wait(&full[s], (it / STAGES) & 1);
           if (!ok) break;
           tc_fence_after();
           const uint32_t a0 = smem_u32(smem + s * STAGE_BYTES), b0 = a0 + 2 * A_STAGE;
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
+#pragma unroll 1
+          for (int h = 0; h < p.halves; ++h)
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k)
-              umma_bf16(acc, umma_desc(a0 + h * A_STAGE + k * 32), umma_desc(b0 + k * 32), (kb | h | k) != 0);
+              umma_bf16(acc, umma_desc(a0 + h * A_STAGE + k * 32), umma_desc(b0 + k * 32), Tile<TN>::IDESC, (kb | h | k) != 0);
           umma_commit(&empty[s]);  // the stage is free once these MMAs have read it
         }
         if (ok) umma_commit(&tfull[buf]);
@@ -254,7 +269,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
       ok = mbar_wait(&tfull[buf], (tc >> 1) & 1);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t acc = tmem_d + buf * BN + ((uint32_t)(q * 32) << 16);
+      const uint32_t acc = tmem_d + buf * TN + ((uint32_t)(q * 32) << 16);
       const int m = mt * BM + row;
       int slot = -1, frame = 0;
       if (p.mode != 0 && m < p.M) {  // the piece that holds row m: the last one that starts at or before it
@@ -268,8 +283,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
         frame = m - pc.x;
         if (frame >= 0 && frame < pc.y && frame < p.T && pc.z >= 0 && pc.z < p.S1) slot = pc.z;
       }
-      for (int c0 = 0; c0 < BN; c0 += 64) {  // warp-uniform trip count: the tensor-memory loads are collective
-        const int n0 = nt * BN + c0;
+      for (int c0 = 0; c0 < TN; c0 += 64) {  // warp-uniform trip count: the tensor-memory loads are collective
+        const int n0 = nt * TN + c0;
         float v[64];
         tmem_ld64(acc + c0, v);
         if (p.bias) {
@@ -296,7 +311,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
                   make_uint4(pack_bf16(v[8 * c], v[8 * c + 1]), pack_bf16(v[8 * c + 2], v[8 * c + 3]),
                              pack_bf16(v[8 * c + 4], v[8 * c + 5]), pack_bf16(v[8 * c + 6], v[8 * c + 7]));
           }
-        } else {
+        } else if constexpr (TN == BN) {
           // int8: the vector's absmax over its D = 64 or 128 channels after rounding to bf16
           float mx = 0.f;
 #pragma unroll
@@ -340,19 +355,27 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_gemm_kernel(const GemmArg
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "n"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "n"(Tile<TN>::TMEM_COLS) : "memory");
   }
 }
 
 // fp32 rows (m, k) -> the operand image [ceil(m / 128)][2 k / 64][128 rows x 128 B, swizzled]: high halves in the first
-// k / 64 blocks of a row tile, low halves in the last; rows past m are zero. One thread per 8 values.
-__global__ void pack_rows_kernel(const float* __restrict__ x, int m, int k, int ldx, unsigned char* __restrict__ out) {
+// k / 64 blocks of a row tile, low halves in the last; rows past m are zero. One thread per 8 values. bf16 rows are their
+// own high halves; the low ones are not written.
+template <class X>
+__global__ void pack_rows_kernel(const X* __restrict__ x, int m, int k, int ldx, unsigned char* __restrict__ out) {
+  pdl_trigger();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int cpr = k / 8, mp = (m + BM - 1) / BM * BM;
   if (i >= (size_t)mp * cpr) return;
   const int r = (int)(i / cpr), c = (int)(i % cpr), kb = c >> 3, chunk = c & 7;
   uint32_t h[4] = {0, 0, 0, 0}, l[4] = {0, 0, 0, 0};
-  if (r < m) {
+  if constexpr (sizeof(X) == 2) {
+    if (r < m) {
+      const uint4 a = *reinterpret_cast<const uint4*>(x + (size_t)r * ldx + c * 8);
+      h[0] = a.x, h[1] = a.y, h[2] = a.z, h[3] = a.w;
+    }
+  } else if (r < m) {
     const float4 a = *reinterpret_cast<const float4*>(x + (size_t)r * ldx + c * 8);
     const float4 b = *reinterpret_cast<const float4*>(x + (size_t)r * ldx + c * 8 + 4);
     const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -365,7 +388,19 @@ __global__ void pack_rows_kernel(const float* __restrict__ x, int m, int k, int 
   const int nkb = k / BK;
   unsigned char* tile = out + (size_t)(r / BM) * (2 * nkb) * A_STAGE;
   *reinterpret_cast<uint4*>(tile + (size_t)kb * A_STAGE + swz(r % BM, chunk)) = make_uint4(h[0], h[1], h[2], h[3]);
-  *reinterpret_cast<uint4*>(tile + (size_t)(nkb + kb) * A_STAGE + swz(r % BM, chunk)) = make_uint4(l[0], l[1], l[2], l[3]);
+  if constexpr (sizeof(X) == 4)
+    *reinterpret_cast<uint4*>(tile + (size_t)(nkb + kb) * A_STAGE + swz(r % BM, chunk)) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+template <int TN>
+int launch_gemm(const GemmArgs& a, int sms, cudaStream_t stream) {
+  constexpr int BYTES = Tile<TN>::SMEM_BYTES;
+  cudaError_t e = cudaFuncSetAttribute(prefill_gemm_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+  if (e != cudaSuccess) return fail(B200DEC_ECUDA, "prefill_gemm: smem attribute: %s", cudaGetErrorString(e));
+  const int tiles = ((a.M + BM - 1) / BM) * (a.N / TN);
+  e = launch_kernel(prefill_gemm_kernel<TN>, dim3(tiles < sms ? tiles : sms), dim3(NTHREADS), BYTES, stream, 0, true, a);
+  if (e != cudaSuccess) return fail(B200DEC_ECUDA, "prefill_gemm launch: %s", cudaGetErrorString(e));
+  return 0;
 }
 
 // bf16 weights (n, k) row-major -> the weight image [n / 256][k / 64][256 rows x 128 B, swizzled]; one thread per 16 B
@@ -374,7 +409,7 @@ __global__ void tile_weight_kernel(const uint4* __restrict__ w, int n, int k, un
   const int cpr = k / 8;
   if (i >= (size_t)n * cpr) return;
   const int r = (int)(i / cpr), c = (int)(i % cpr), kb = c >> 3, chunk = c & 7;
-  *reinterpret_cast<uint4*>(out + ((size_t)(r / BN) * (k / BK) + kb) * B_STAGE + swz(r % BN, chunk)) = w[i];
+  *reinterpret_cast<uint4*>(out + ((size_t)(r / BN) * (k / BK) + kb) * B_BLOCK + swz(r % BN, chunk)) = w[i];
 }
 
 }  // namespace
@@ -395,6 +430,16 @@ int b200dec_prefill_pack_rows(const float* x, int m, int k, int ldx, void* image
   return check_launch("prefill_pack_rows");
 }
 
+int b200dec_prefill_pack_rows_bf16(const void* x, int m, int k, int ldx, void* image, void* stream) {
+  B200_REQUIRE(x && image && m >= 1 && k >= BK && k % BK == 0 && ldx >= k && ldx % 8 == 0 && ((uintptr_t)x & 15) == 0 &&
+                   ((uintptr_t)image & 1023) == 0, "prefill_pack_rows_bf16: m %d k %d ldx %d (k a multiple of 64, rows "
+               "16-byte, image 1 KB aligned)", m, k, ldx);
+  const size_t total = (size_t)((m + BM - 1) / BM) * BM * (k / 8);
+  pack_rows_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, m, k, ldx,
+                                                                                      (unsigned char*)image);
+  return check_launch("prefill_pack_rows_bf16");
+}
+
 int b200dec_prefill_tile_weight(const void* w_bf16, int n, int k, void* image, void* stream) {
   B200_REQUIRE(w_bf16 && image && n >= BN && n % BN == 0 && k >= BK && k % BK == 0 && ((uintptr_t)w_bf16 & 15) == 0 &&
                    ((uintptr_t)image & 1023) == 0, "prefill_tile_weight: (%d, %d) must be multiples of (256, 64)", n, k);
@@ -412,6 +457,8 @@ int b200dec_prefill_gemm(const void* rows_image, int m, int k, const void* weigh
   B200_REQUIRE(m >= 1 && k >= BK && k % BK == 0 && n >= BN && n % BN == 0, "prefill_gemm: m %d k %d n %d", m, k, n);
   B200_REQUIRE(((uintptr_t)rows_image & 1023) == 0 && ((uintptr_t)weight_image & 1023) == 0 && ((uintptr_t)bias & 15) == 0,
                "prefill_gemm: the operand images must be 1 KB aligned, the bias 16-byte aligned");
+  const int halves = (mode & B200DEC_PREFILL_HIGH_ROWS) ? 1 : 2;
+  mode &= ~B200DEC_PREFILL_HIGH_ROWS;
   B200_REQUIRE(mode >= 0 && mode <= 2, "prefill_gemm: mode %d", mode);
   if (mode == 0) {
     B200_REQUIRE(next_image && ((uintptr_t)next_image & 1023) == 0, "prefill_gemm: mode 0 writes the next operand image");
@@ -423,18 +470,18 @@ int b200dec_prefill_gemm(const void* rows_image, int m, int k, const void* weigh
                  layers, heads, head_dim);
     B200_REQUIRE(mode != 2 || (ck_scale && cv_scale), "prefill_gemm: int8 caches need their scales");
   }
-  cudaError_t e = cudaFuncSetAttribute(prefill_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  if (e != cudaSuccess) return fail(B200DEC_ECUDA, "prefill_gemm: smem attribute: %s", cudaGetErrorString(e));
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int tiles = ((m + BM - 1) / BM) * (n / BN);
-  GemmArgs a{(const unsigned char*)rows_image, (const unsigned char*)weight_image, bias, m, n, k, mode,
+  GemmArgs a{(const unsigned char*)rows_image, (const unsigned char*)weight_image, bias, m, n, k, mode, halves,
              (unsigned char*)next_image, (const int4*)pieces, n_pieces, ck, cv, ck_scale, cv_scale, slots_plus_1, heads,
              head_dim, frames, status};
-  e = launch_kernel(prefill_gemm_kernel, dim3(tiles < sms ? tiles : sms), dim3(NTHREADS), SMEM_BYTES,
-                    (cudaStream_t)stream, 0, false, a);
-  if (e != cudaSuccess) return fail(B200DEC_ECUDA, "prefill_gemm launch: %s", cudaGetErrorString(e));
-  return 0;
+  // A few clips' first product (1024 channels: 4 wide tiles per 128 rows) leaves most SMs idle, and each CTA is bound by
+  // what it copies: 64 KB per 64 k of a wide tile, 40 KB of a narrow one. Narrow as long as that is one wave; beyond it
+  // the rows would be copied again by every further wave. Both products, us on the device with narrow / wide tiles in the first:
+  // 30.6 / 35.8 at 175 frames, 53.0 / 57.2 at 640, 67.0 / 72.0 at 1152 (one wave of 144). With the products launched behind
+  // one another programmatically and bf16 rows packed as they are, a prefill of 175 bf16 frames went from 40.6 to 28.1.
+  if (mode == 0 && ((m + BM - 1) / BM) * (n / 64) <= sms) return launch_gemm<64>(a, sms, (cudaStream_t)stream);
+  return launch_gemm<BN>(a, sms, (cudaStream_t)stream);
 }
 
 }  // extern "C"

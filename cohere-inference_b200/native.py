@@ -19,6 +19,7 @@ A_F16, A_F32_SPLIT, A_F16_ROWS16 = 0, 1, 2
 OUT_F16, OUT_F32, OUT_F32_ADD = 0, 1, 2
 ACT_NONE, ACT_RELU, ACT_GELU = 0, 1, 2
 ST_TOKEN_RANGE, ST_POS_RANGE, ST_FRAMES_RANGE, ST_SLOT_RANGE, ST_TIMEOUT = 1, 2, 4, 8, 16
+PREFILL_HIGH_ROWS = 8
 
 vp, i32, i64, f32 = C.c_void_p, C.c_int32, C.c_int64, C.c_float
 
@@ -114,6 +115,7 @@ PROTOTYPES = {
     "b200dec_scatter_kv": (C.c_int, [vp, vp, vp, vp, vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, vp]),
     "b200dec_prefill_rows_bytes": (i64, [C.c_int, C.c_int]),
     "b200dec_prefill_pack_rows": (C.c_int, [vp, C.c_int, C.c_int, C.c_int, vp, vp]),
+    "b200dec_prefill_pack_rows_bf16": (C.c_int, [vp, C.c_int, C.c_int, C.c_int, vp, vp]),
     "b200dec_prefill_tile_weight": (C.c_int, [vp, C.c_int, C.c_int, vp, vp]),
     "b200dec_prefill_gemm": (C.c_int, [vp, C.c_int, C.c_int, vp, vp, C.c_int, C.c_int, vp, vp, C.c_int, vp, vp, vp, vp,
                                        C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp]),

@@ -408,6 +408,11 @@ class StreamDecoder:
         # kernel (admit() clears it on the host, as the reference does)
         p.flags_host = self.flags.data_ptr()
         self.plan = p
+        # what every fill_cross hands to its two products
+        weight = lambda w: (w.k, nv.ptr(w.image), nv.ptr(w.bias), w.n)  # noqa: E731
+        self._prefill_args = (nv.ptr(self.status), weight(self.proj), weight(self.cross),
+                              (*(nv.ptr(t) for t in (self.cross_k, self.cross_v, self.cross_ks, self.cross_vs)), L,
+                               self.slots + 1, self.h, self.d, self.frames))
 
     def _fused_workspaces(self, fused_rows: int) -> dict[int, torch.Tensor]:
         """Exchange buffers of the buckets whose step is one kernel, by rows (their initial state: reset())."""
@@ -552,18 +557,20 @@ class StreamDecoder:
                 return b
         raise ValueError(f"{rows} rows exceed the largest bucket {self.buckets[-1]}")
 
-    def _stage(self, values: np.ndarray, dst: torch.Tensor, stream: torch.cuda.Stream | None = None) -> None:
-        """int32 values -> dst (device int32, at least as long) through the pinned ring, on `stream` (default: the
-        decoder stream)."""
-        stream = stream or self.stream
+    def _stage(self, values: np.ndarray, dst: torch.Tensor) -> None:
+        """int32 values -> dst (device int32, at least as long) through the pinned ring, on the decoder stream."""
+        with torch.cuda.stream(self.stream):
+            self._stage_here(values, dst, self.stream)
+
+    def _stage_here(self, values: np.ndarray, dst: torch.Tensor, stream: torch.cuda.Stream) -> None:
+        """The same on `stream`, which is the current one."""
         n = int(values.size)
         buf, ev = self._ring[self._ring_at]
         self._ring_at = (self._ring_at + 1) % len(self._ring)
         ev.synchronize()  # the copy that last used this buffer (several calls ago) has long finished
         buf.numpy()[:n] = values.reshape(-1)
-        with torch.cuda.stream(stream):
-            dst[:n].copy_(buf[:n], non_blocking=True)
-            ev.record(stream)
+        dst[:n].copy_(buf[:n], non_blocking=True)
+        ev.record(stream)
 
     @torch.no_grad()
     def fill_cross(self, hidden: torch.Tensor, lengths: list[int], slots: list[int]) -> None:
@@ -578,30 +585,34 @@ class StreamDecoder:
         if m == 0:
             return
         lib, cur = nv.lib(), torch.cuda.current_stream()
-        x = hidden.float().contiguous()
+        x, high = hidden.contiguous(), 0
+        if hidden.dtype == torch.bfloat16 and x.is_cuda:
+            high = nv.PREFILL_HIGH_ROWS
+            x = x if x.data_ptr() % 16 == 0 else x.clone()
+        else:
+            x = x.float()
         pieces = np.zeros((len(slots), 4), np.int32)
-        pieces[:, 0] = np.concatenate([[0], np.cumsum(lengths[:-1])])
+        pieces[1:, 0] = np.cumsum(lengths[:-1])
         pieces[:, 1], pieces[:, 2] = lengths, slots
-        table = torch.empty(pieces.size, dtype=torch.int32, device=self.device)
+        # the two operand images, on a 1 KB boundary, and the table of pieces
+        n0, n1 = lib.b200dec_prefill_rows_bytes(m, self.proj.k), lib.b200dec_prefill_rows_bytes(m, self.proj.n)
+        work = torch.empty(1024 + n0 + n1 + pieces.nbytes, dtype=torch.uint8, device=self.device)
+        pad = -work.data_ptr() % 1024
+        a0 = work.data_ptr() + pad
+        a1 = a0 + n0
+        table = work[pad + n0 + n1:pad + n0 + n1 + pieces.nbytes].view(torch.int32)
         if pieces.size <= self._ring[0][0].numel():
-            self._stage(pieces, table, cur)
+            self._stage_here(pieces, table, cur)
         else:
             table.copy_(torch.from_numpy(pieces.reshape(-1)))
-        img = lambda k: torch.empty(lib.b200dec_prefill_rows_bytes(m, k) + 1024, dtype=torch.uint8, device=self.device)  # noqa: E731
-        aligned = lambda t: t.data_ptr() + (-t.data_ptr()) % 1024  # noqa: E731
-        a0, a1 = img(self.proj.k), img(self.proj.n)
-        s = cur.cuda_stream
-        nv.check(lib.b200dec_prefill_pack_rows(nv.ptr(x), m, self.proj.k, x.shape[1], aligned(a0), s))
-        nv.check(lib.b200dec_prefill_gemm(aligned(a0), m, self.proj.k, nv.ptr(self.proj.image), nv.ptr(self.proj.bias),
-                                          self.proj.n, 0, aligned(a1), None, 0, None, None, None, None, 0, 0, 0, 0, 0,
-                                          nv.ptr(self.status), s))
-        nv.check(lib.b200dec_prefill_gemm(aligned(a1), m, self.cross.k, nv.ptr(self.cross.image), nv.ptr(self.cross.bias),
-                                          self.cross.n, 2 if self.kv_int8 else 1, None, nv.ptr(table), len(slots),
-                                          nv.ptr(self.cross_k), nv.ptr(self.cross_v), nv.ptr(self.cross_ks),
-                                          nv.ptr(self.cross_vs), len(self.layers), self.slots + 1, self.h, self.d,
-                                          self.frames, nv.ptr(self.status), s))
-        for t in (x, table, a0, a1):
-            t.record_stream(cur)
+        s, (status, first, second, caches) = cur.cuda_stream, self._prefill_args
+        pack = lib.b200dec_prefill_pack_rows_bf16 if high else lib.b200dec_prefill_pack_rows
+        nv.check(pack(nv.ptr(x), m, self.proj.k, x.shape[1], a0, s))
+        nv.check(lib.b200dec_prefill_gemm(a0, m, *first, 0 | high, a1, None, 0, None, None, None, None, 0, 0, 0, 0, 0,
+                                          status, s))
+        nv.check(lib.b200dec_prefill_gemm(a1, m, *second, 2 if self.kv_int8 else 1, None, a1 + n1, len(slots), *caches,
+                                          status, s))
+        hidden.record_stream(cur)  # the others come from this stream's pool
 
     def admit(self, slots: list[int], prompts: list, frames: list[int], max_new: list[int] | None = None) -> None:
         """Start decoding in `slots`: each gets its prompt (fed token by token as forced choices), its number of

@@ -348,6 +348,9 @@ int b200dec_read_probe(const void* src, int ctas, int64_t bytes_per_cta, int32_t
 int64_t b200dec_prefill_rows_bytes(int m, int k); /* bytes of the image of m fp32 rows of k values (k % 64 == 0) */
 /* x (m, ldx) fp32 -> its image (1 KB aligned, b200dec_prefill_rows_bytes(m, k) bytes). */
 int b200dec_prefill_pack_rows(const float* x, int m, int k, int ldx, void* image, void* stream);
+/* The same for bf16 rows: they are their own high halves; the image's low ones are not written, and a product over such
+ * an image is asked for with B200DEC_PREFILL_HIGH_ROWS. */
+int b200dec_prefill_pack_rows_bf16(const void* x, int m, int k, int ldx, void* image, void* stream);
 /* w (n, k) bf16 row-major (n % 256 == 0, k % 64 == 0) -> its image (1 KB aligned, n * k * 2 bytes); init time. */
 int b200dec_prefill_tile_weight(const void* w_bf16, int n, int k, void* image, void* stream);
 /* mode 0: next_image = the image of the m result rows (n values each) for the next product.
@@ -357,7 +360,9 @@ int b200dec_prefill_tile_weight(const void* w_bf16, int n, int k, void* image, v
  *   frames, head_dim) of keys (kv = 0) or values. Rows outside every piece or past the cache are dropped.
  * mode 2: the same into int8 caches with one fp32 scale per head vector (layers, slots_plus_1, heads, frames),
  *   quantised as b200dec_scatter_kv_q8 does.
+ * mode | B200DEC_PREFILL_HIGH_ROWS: the low halves of A are zero and the image does not hold them.
  * status receives B200DEC_ST_TIMEOUT if a bounded wait inside the kernel ran out. */
+#define B200DEC_PREFILL_HIGH_ROWS 8
 int b200dec_prefill_gemm(const void* rows_image, int m, int k, const void* weight_image, const float* bias, int n,
                          int mode, void* next_image, const int32_t* pieces, int n_pieces, void* ck, void* cv,
                          float* ck_scale, float* cv_scale, int layers, int slots_plus_1, int heads, int head_dim,

@@ -503,3 +503,24 @@ def test_decoder_from_a_checkpoint_directory(tmp_path, style, shards):
     assert (again.h, again.d, again.proj.k) == (8, 128, 1280)
     got, _ = _run_teacher_forced(again, memory, prompts, 5)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("lens", [[1], [127, 1], [129], [300, 375, 375, 103], [300, 375, 375, 375]])
+def test_prefill_of_bf16_frames_is_that_of_their_fp32_values(lens):
+    """bf16 encoder frames go into the prefill as they are (no low halves: they are zero); fp32 frames of the same values
+    take the two halves. Same bits in the caches: up to one row tile, past it, and on both sides of the row count at which
+    the first product goes from narrow channel tiles to wide ones (1152 frames). A view that starts off a 16-byte
+    boundary, as a slice of a packed buffer may."""
+    dec = _decoder(_two_layers(16), slots=4, max_new_tokens=8, max_prompt=8, max_audio_s=30.0, eos=-1, int8=True)
+    g = torch.Generator(device="cuda").manual_seed(len(lens))
+    flat = torch.randn(sum(lens) * 1024 + 1, device="cuda", generator=g).to(torch.bfloat16)
+    got = []
+    for frames in (flat[1:].view(-1, 1024), flat[1:].view(-1, 1024).float()):
+        with torch.cuda.stream(dec.stream):
+            dec.cross_k.zero_(), dec.cross_v.zero_()
+            dec.stream.wait_stream(torch.cuda.default_stream())
+            dec.fill_cross(frames, lens, list(range(len(lens))))
+        dec.check_status()
+        got.append((dec.cross_k.clone(), dec.cross_v.clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert all(bool(got[0][0][:, i, :, :n].any()) for i, n in enumerate(lens))
