@@ -515,6 +515,66 @@ __global__ void __launch_bounds__(NTHREADS, 7) attention_pair_kernel(const AttnA
   }
 }
 
+// ---- middling batches: a row's keys cut into spans, one CTA of a cluster each -------------------------------------------
+//
+// With a few hundred (row, head) items one CTA per item leaves SMs idle, and a long row's CTA decides when the kernel ends.
+// A cluster of up to four CTAs takes an item: as many of them as the row has SPAN_KEYS keys for share its keys, the others
+// leave; the first one gets the others' partials (max, sum, output) through distributed shared memory behind one cluster
+// barrier. Rows come from the schedule, longest first, read before the wait as in the paired kernel. Against the split of
+// attention_kernel this has no workspace, no counter, no fence, and a short row is not split at all. A step of 32 rows, 8 x
+// 128 heads, int8 caches, 50 / 50-375 / 375 frames at position 10 / 150 / 440: 310 / 345 / 387 us, with the split 358 /
+// 389 / 431; bf16 caches 296 / 357 / 422 against 338 / 411 / 475 (rows paired: 288 / 413 / 570).
+constexpr int SPAN_MAX = 4, SPAN_KEYS = 64;
+
+template <int D, bool SELF, bool Q8>
+__global__ void __launch_bounds__(NTHREADS, 7) attention_span_kernel(const AttnArgs p) {
+  constexpr int NG = NTHREADS / (Q8 ? D / Q8_LANE_DIMS : D / 8);
+  __shared__ float s_m[NG], s_l[NG];
+  __shared__ float s_acc[NG][D + 4];
+  __shared__ float s_peer[SPAN_MAX - 1][D + 2];  // CTA 0: the others' partials
+
+  cluster_arrive_entry();
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  const int4 row = __ldcg(reinterpret_cast<const int4*>(p.sched) + blockIdx.z);
+  pdl_wait();
+  const int r = row.x, s = row.y, n = row.z;
+  const int spans = max(1, min((int)gridDim.x, (n + SPAN_KEYS - 1) / SPAN_KEYS));
+  if (rank >= spans) {
+    pdl_trigger();
+    if (spans > 1) {
+      cluster_wait_entry();
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");  // the others' barrier below counts every CTA
+    }
+    return;
+  }
+  const int chunk = ((n + spans - 1) / spans + 15) & ~15, start = rank * chunk, end = min(n, start + chunk);
+  float M, L, O;
+  attend_pass<D, SELF, Q8>(p, r, s, h, n, start, end, rank == 0, s_m, s_l, s_acc, M, L, O);
+  pdl_trigger();  // late: see attention_kernel
+  if (spans > 1) {
+    cluster_wait_entry();  // CTA 0 has started
+    if (rank > 0) {
+      float* peer = cluster.map_shared_rank(&s_peer[0][0], 0) + (rank - 1) * (D + 2);
+      if (tid < D) peer[tid] = O;
+      if (tid == 0) peer[D] = M, peer[D + 1] = L;
+    }
+    cluster.sync();
+    if (rank > 0) return;
+    if (tid < D) {
+      float mm = M;
+      for (int i = 0; i < spans - 1; ++i) mm = fmaxf(mm, s_peer[i][D]);
+      const float w0 = ex2(M - mm);
+      L *= w0, O *= w0;
+      for (int i = 0; i < spans - 1; ++i) {
+        const float w = ex2(s_peer[i][D] - mm);
+        L += w * s_peer[i][D + 1], O += w * s_peer[i][tid];
+      }
+    }
+  }
+  if (tid < D) store_out<D>(p, r, h, O / L);
+}
+
 int pick_splits(int rows, int heads, int cap) {
   // enough CTAs for every SM to hold several, but at least ~32 keys per split
   const int items = rows * heads;
@@ -579,9 +639,46 @@ int run_attention(const char* what, int self, const int32_t* active, const float
   return 0;
 }
 
+template <bool Q8>
+cudaError_t launch_spans(int head_dim, int self, dim3 grid, cudaStream_t s, int pdl, const AttnArgs& p) {
+#define B200_SPAN_CASE(D_, SELF_)                  \
+  if (head_dim == D_ && (self != 0) == SELF_)      \
+    return launch_kernel(attention_span_kernel<D_, SELF_, Q8>, grid, dim3(NTHREADS), 0, s, grid.x, pdl, p);
+  B200_SPAN_CASE(64, true)
+  B200_SPAN_CASE(64, false)
+  B200_SPAN_CASE(128, true)
+  B200_SPAN_CASE(128, false)
+#undef B200_SPAN_CASE
+  return cudaErrorInvalidValue;
+}
+
 }  // namespace
 
 extern "C" {
+
+int b200dec_attention_spans(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache,
+                            float* kscale, float* vscale, int heads, int head_dim, int cap, float scale, void* out,
+                            int out_kind, int rows, int pdl, void* stream) {
+  B200_REQUIRE(sched && q && kcache && vcache && out, "attention_spans: null pointer");
+  B200_REQUIRE((kscale == nullptr) == (vscale == nullptr), "attention_spans: key and value scales go together");
+  B200_REQUIRE(head_dim == 64 || head_dim == 128, "attention_spans: head_dim %d (64 or 128)", head_dim);
+  B200_REQUIRE(rows >= 1 && rows <= 65535 && heads >= 1 && heads <= 65535 && cap >= 1,
+               "attention_spans: rows %d heads %d cap %d", rows, heads, cap);
+  B200_REQUIRE(ldq % 4 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)kcache & 15) == 0 &&
+                   ((uintptr_t)vcache & 15) == 0 && ((uintptr_t)sched & 15) == 0, "attention_spans: alignment");
+  B200_REQUIRE(out_kind == B200DEC_OUT_F16 || out_kind == B200DEC_OUT_F32, "attention_spans: out_kind");
+  AttnArgs p{};
+  p.q = q, p.k = (__nv_bfloat16*)kcache, p.v = (__nv_bfloat16*)vcache, p.ks = kscale, p.vs = vscale;
+  p.sched = sched, p.out = out, p.ldq = ldq, p.H = heads, p.cap = cap, p.out_kind = out_kind, p.rows = rows;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  const int64_t items = (int64_t)rows * heads;
+  const int want = (int)((4 * 148 + items - 1) / items);  // four CTAs per SM
+  const dim3 grid(want < SPAN_MAX ? want : SPAN_MAX, heads, rows);
+  const cudaError_t e = kscale ? launch_spans<true>(head_dim, self, grid, (cudaStream_t)stream, pdl, p)
+                               : launch_spans<false>(head_dim, self, grid, (cudaStream_t)stream, pdl, p);
+  if (e != cudaSuccess) return fail(B200DEC_ECUDA, "attention_spans launch: %s", cudaGetErrorString(e));
+  return 0;
+}
 
 int64_t b200dec_attention_scratch_floats(int rows, int heads, int head_dim) {
   return (int64_t)rows * heads * MAX_SPLITS * (head_dim + 2);

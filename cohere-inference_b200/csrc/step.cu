@@ -144,8 +144,10 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
   // a large batch: the rows are ranked by length once (an extra CTA of the embedding kernel) and the attention
   // kernels pair long rows with short ones from the two tables
   const bool paired = !pl->attn_ring && pl->sched_self && pl->sched_cross && rows * pl->heads >= 512 && rows <= 256;
-  int32_t* sched_self = paired ? pl->sched_self + 4 * row0 : nullptr;
-  int32_t* sched_cross = paired ? pl->sched_cross + 4 * row0 : nullptr;
+  // a middling one takes them from the tables too, longest first, each row's keys shared by a cluster
+  const bool spans = !pl->attn_ring && pl->sched_self && pl->sched_cross && !paired && rows * pl->heads >= 128;
+  int32_t* sched_self = paired || spans ? pl->sched_self + 4 * row0 : nullptr;
+  int32_t* sched_cross = paired || spans ? pl->sched_cross + 4 * row0 : nullptr;
 
   // Prefetch of the attention launches' caches into L2 by the output projections (common.cuh, KvPrefetch): the budget
   // in keys per launch; one key of a row is 2 (key, value) x heads x vec_bytes bytes.
@@ -183,7 +185,11 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
     // projections left out (classes) the first self-attention would follow the embedding directly and the two CTAs of
     // a pair could see different versions of an entry and disagree on their hand-off: it is then launched plainly.
     const int pdl_self = (i == 0 && !(want & 2)) ? 0 : pdl_attn;
-    if (pl->kv_int8 && paired)
+    if (spans)
+      B200_TRY_IN(4, b200dec_attention_spans(1, sched_self, qkv, 3 * hd, ly.self_k, ly.self_v,
+                                             pl->kv_int8 ? ly.self_ks : nullptr, pl->kv_int8 ? ly.self_vs : nullptr,
+                                             pl->heads, pl->head_dim, pl->seq, scale, att, ok_a, rows, pdl_self, stream));
+    else if (pl->kv_int8 && paired)
       B200_TRY_IN(4, b200dec_attention_paired_q8(1, sched_self, qkv, 3 * hd, ly.self_k, ly.self_v, ly.self_ks, ly.self_vs,
                                            pl->heads, pl->head_dim, pl->seq, scale, att, ok_a, rows, pdl_self, stream));
     else if (pl->kv_int8)
@@ -201,7 +207,11 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
                          pdl_after, stream, &p2, &f_cross));
     B200_TRY_IN(2, linear_impl(&ly.cq, ln_src, ln_kind, &ly.ln2, D_MODEL, rows, cq, B200DEC_OUT_F32, hd, B200DEC_ACT_NONE, pdl,
                          stream, &r2, nullptr));
-    if (pl->kv_int8 && paired)
+    if (spans)
+      B200_TRY_IN(4, b200dec_attention_spans(0, sched_cross, cq, hd, (void*)ly.cross_k, (void*)ly.cross_v,
+                                             pl->kv_int8 ? ly.cross_ks : nullptr, pl->kv_int8 ? ly.cross_vs : nullptr,
+                                             pl->heads, pl->head_dim, pl->frames, scale, att, ok_a, rows, pdl_attn, stream));
+    else if (pl->kv_int8 && paired)
       B200_TRY_IN(4, b200dec_attention_paired_q8(0, sched_cross, cq, hd, (void*)ly.cross_k, (void*)ly.cross_v, ly.cross_ks,
                                            ly.cross_vs, pl->heads, pl->head_dim, pl->frames, scale, att, ok_a, rows,
                                            pdl_attn, stream));

@@ -108,6 +108,8 @@ PROTOTYPES = {
     "b200dec_row_schedule": (C.c_int, [vp, vp, vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp]),
     "b200dec_attention_paired": (C.c_int, [C.c_int, vp, vp, C.c_int, vp, vp, C.c_int, C.c_int, C.c_int, f32, vp,
                                            C.c_int, C.c_int, C.c_int, vp]),
+    "b200dec_attention_spans": (C.c_int, [C.c_int, vp, vp, C.c_int, vp, vp, vp, vp, C.c_int, C.c_int, C.c_int, f32, vp,
+                                          C.c_int, C.c_int, C.c_int, vp]),
     "b200dec_attention_ring": (C.c_int, [C.c_int, vp, vp, C.c_int, vp, vp, vp, C.c_int, C.c_int, C.c_int, C.c_int, f32,
                                          vp, C.c_int, C.c_int, vp, vp, vp, C.c_int, vp]),
     "b200dec_attention_static": (C.c_int, [C.c_int, vp, vp, C.c_int, vp, vp, vp, C.c_int, C.c_int, C.c_int, C.c_int,

@@ -138,7 +138,7 @@ typedef struct b200dec_plan {
   void* xh;             /* (max rows, 1024) fp16: the residual stream times the next LayerNorm's gamma, the operand of
                            the LayerNorm-folding projections (a_kind F16 only); NULL: they convert the fp32 rows */
   float* ln_stats;      /* (max rows, 128, 2) partial row sums that go with xh (see b200dec_ln_link) */
-  int32_t* sched_self;  /* (max rows, 4) row schedules for b200dec_attention_paired, 16-byte aligned; both NULL: */
+  int32_t* sched_self;  /* (max rows, 4) row schedules for b200dec_attention_paired and _spans, 16-byte aligned; both NULL: */
   int32_t* sched_cross; /* the step uses b200dec_attention for every batch size */
   /* optional recording (tests, teacher forcing); NULL in production */
   float* logits;       /* (rows, vocab) */
@@ -302,6 +302,12 @@ int b200dec_attention_paired(int self, const int32_t* sched, const float* q, int
 int b200dec_attention_paired_q8(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache,
                                 float* kscale, float* vscale, int heads, int head_dim, int cap, float scale, void* out,
                                 int out_kind, int rows, int pdl, void* stream);
+/* b200dec_attention for a middling batch (128 <= rows * heads < 512 is where it pays), reading the rows from a schedule as
+ * b200dec_attention_paired does (the same rule for pdl): a cluster of up to four CTAs takes a (row, head), as many of them
+ * as the row has 64 keys for share its keys. kscale, vscale: those of int8 caches, or both NULL for bf16 caches. */
+int b200dec_attention_spans(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache,
+                            float* kscale, float* vscale, int heads, int head_dim, int cap, float scale, void* out,
+                            int out_kind, int rows, int pdl, void* stream);
 /* The same operation, arguments and workspace as b200dec_attention (rows <= 128) by a persistent kernel: two CTAs
  * per SM, one producer lane streaming (row, head) caches through a shared-memory ring with cp.async.bulk and
  * mbarriers, four consumer warps. Smaller footprint per SM; see csrc/attention_ring.cu. */

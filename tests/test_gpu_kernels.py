@@ -647,6 +647,56 @@ def test_attention(nv, H, D, rows, self_, cap, ring):
 
 
 @pytest.mark.parametrize("H,D", [(16, 64), (8, 128)])
+@pytest.mark.parametrize("rows", [17, 24, 31])  # four, three and two CTAs per (row, head) of both head counts
+@pytest.mark.parametrize("self_", [0, 1])
+@pytest.mark.parametrize("q8", [False, True])
+def test_attention_spans_against_one_cta_per_row(nv, H, D, rows, self_, q8):
+    """A row's keys shared by a cluster: the same output as the kernel that gives every row one CTA, and the same bytes
+    appended. Lengths on both sides of every number of spans (64 keys each) and of the 16 keys a span is rounded to. bf16
+    caches: fp32 sums in another order. int8 caches: the weighted sums run through fp16 pairs whose chains a span
+    shortens, half a unit (2^-11 of the largest value, |v| < 4) per addition of up to cap / 16 = 20 per lane."""
+    cap = 320
+    rng = np.random.default_rng(rows + H + self_)
+    lens = [0 if self_ else 1, 1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 191, 192, 193, 255, 256, 257, cap - 1]
+    n = np.array([lens[i % len(lens)] for i in range(rows + 2)], np.int32)
+    active = rng.permutation(rows + 1)[:rows].astype(np.int32)
+    ld = 3 * H * D if self_ else H * D
+    q_d, a_d, n_d = cuda(rng.standard_normal((rows, ld)).astype(np.float32)), cuda(active), cuda(n)
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    kv = [torch.randn(rows + 2, H, cap, D, device="cuda", generator=gen) for _ in range(2)]
+    kv = [(t.clamp(-4, 4) * 31).to(torch.int8) if q8 else t.to(torch.bfloat16) for t in kv]
+    sc = [torch.full((rows + 2, H, cap), 1 / 31, device="cuda") if q8 else None for _ in range(2)]
+    lib, scale = nv.lib(), D ** -0.5
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    sched = torch.zeros(rows, 4, dtype=torch.int32, device="cuda")
+    nv.check(lib.b200dec_row_schedule(nv.ptr(a_d), nv.ptr(n_d) if self_ else None, None if self_ else nv.ptr(n_d), rows + 1,
+                                      cap, cap, rows, 0, nv.ptr(sched) if self_ else None,
+                                      None if self_ else nv.ptr(sched), nv.ptr(status), nv.stream_ptr()))
+    got = []
+    for spans in (False, True):
+        (k, v), (ks, vs) = [t.clone() for t in kv], [t.clone() if q8 else None for t in sc]
+        out = torch.full((rows, H * D), 7.0, device="cuda")
+        if spans:
+            nv.check(lib.b200dec_attention_spans(self_, nv.ptr(sched), nv.ptr(q_d), ld, nv.ptr(k), nv.ptr(v), nv.ptr(ks),
+                                                 nv.ptr(vs), H, D, cap, scale, nv.ptr(out), nv.OUT_F32, rows, 0,
+                                                 nv.stream_ptr()))
+        elif q8:
+            nv.check(lib.b200dec_attention_q8(self_, nv.ptr(a_d), nv.ptr(q_d), ld, nv.ptr(k), nv.ptr(v), nv.ptr(ks),
+                                              nv.ptr(vs), nv.ptr(n_d), rows + 1, H, D, cap, scale, nv.ptr(out), nv.OUT_F32,
+                                              rows, None, None, nv.ptr(status), 0, nv.stream_ptr()))
+        else:
+            nv.check(lib.b200dec_attention(self_, nv.ptr(a_d), nv.ptr(q_d), ld, nv.ptr(k), nv.ptr(v), nv.ptr(n_d),
+                                           rows + 1, H, D, cap, scale, nv.ptr(out), nv.OUT_F32, rows, None, None,
+                                           nv.ptr(status), 0, nv.stream_ptr()))
+        got.append((out, k, v) + ((ks, vs) if q8 else ()))
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert float((got[0][0] - got[1][0]).abs().max()) <= (20 * 4 * 2.0 ** -11 if q8 else 2e-5)
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H,D", [(16, 64), (8, 128)])
 @pytest.mark.parametrize("rows", [2, 41, 64])
 @pytest.mark.parametrize("self_", [0, 1])
 def test_row_schedule_and_paired_attention(nv, H, D, rows, self_):
