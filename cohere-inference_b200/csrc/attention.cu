@@ -515,13 +515,14 @@ __global__ void __launch_bounds__(NTHREADS, 7) attention_pair_kernel(const AttnA
   }
 }
 
-// ---- middling batches: a row's keys cut into spans, one CTA of a cluster each -------------------------------------------
+// ---- a row's keys cut into spans, one CTA of a cluster each -------------------------------------------------------------
 //
 // With a few hundred (row, head) items one CTA per item leaves SMs idle, and a long row's CTA decides when the kernel ends.
 // A cluster of up to four CTAs takes an item: as many of them as the row has SPAN_KEYS keys for share its keys, the others
 // leave; the first one gets the others' partials (max, sum, output) through distributed shared memory behind one cluster
 // barrier. Rows come from the schedule, longest first, read before the wait as in the paired kernel. Against the split of
-// attention_kernel this has no workspace, no counter, no fence, and a short row is not split at all. A step of 32 rows, 8 x
+// attention_kernel this has no workspace, no counter, no fence, and a short row is not split at all. With more items than
+// fit at once the clusters are single CTAs, and the order alone evens the work out (step.cu has the lines). A step of 32 rows, 8 x
 // 128 heads, int8 caches, 50 / 50-375 / 375 frames at position 10 / 150 / 440: 310 / 345 / 387 us, with the split 358 /
 // 389 / 431; bf16 caches 296 / 357 / 422 against 338 / 411 / 475 (rows paired: 288 / 413 / 570).
 constexpr int SPAN_MAX = 4, SPAN_KEYS = 64;

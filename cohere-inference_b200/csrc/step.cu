@@ -141,19 +141,24 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
   };
 
   const auto attention = pl->attn_ring ? b200dec_attention_ring : b200dec_attention;
-  // a large batch: the rows are ranked by length once (an extra CTA of the embedding kernel) and the attention
-  // kernels pair long rows with short ones from the two tables
-  const bool paired = !pl->attn_ring && pl->sched_self && pl->sched_cross && rows * pl->heads >= 512 && rows <= 256;
-  // a middling one takes them from the tables too, longest first, each row's keys shared by a cluster
-  const bool spans = !pl->attn_ring && pl->sched_self && pl->sched_cross && !paired && rows * pl->heads >= 128;
-  int32_t* sched_self = paired || spans ? pl->sched_self + 4 * row0 : nullptr;
-  int32_t* sched_cross = paired || spans ? pl->sched_cross + 4 * row0 : nullptr;
+  // From 128 (row, head) items on the rows are ranked by length once (an extra CTA of the embedding kernel) and the
+  // attention kernels take them from the two tables, in one of two ways. Below four CTAs per SM's worth of items, a
+  // cluster shares a row's keys (spans); with more than one wave of CTAs (seven per SM) every row has one CTA and the
+  // longest go first, the short ones filling up: the same kernel with clusters of one. In between, where all CTAs are
+  // resident and the longest decides, long rows are paired with short ones. Paired / this way, us a step, ragged rows at
+  // position 30-270: 512 items 477 / 443 (8 x 128, fp16), 371 / 341 (16 x 64, int8 caches); 1536 585 / 543, 559 / 504 and
+  // 2048 669 / 635, 623 / 574 (16 x 64, bf16 / int8 caches); paired the better one at 768 (620 / 666) and 896 (678 / 723).
+  const int items = rows * pl->heads;
+  const bool ranked = !pl->attn_ring && pl->sched_self && pl->sched_cross && items >= 128 && rows <= 256;
+  const bool paired = ranked && items >= 4 * 148 && items <= 7 * 148, spans = ranked && !paired;
+  int32_t* sched_self = ranked ? pl->sched_self + 4 * row0 : nullptr;
+  int32_t* sched_cross = ranked ? pl->sched_cross + 4 * row0 : nullptr;
 
   // Prefetch of the attention launches' caches into L2 by the output projections (common.cuh, KvPrefetch): the budget
   // in keys per launch; one key of a row is 2 (key, value) x heads x vec_bytes bytes.
   const int vec_bytes = pl->head_dim * (pl->kv_int8 ? 1 : 2);
   const int prefetch_keys =
-      paired && pl->kv_prefetch_mb > 0 ? (int)(((long long)pl->kv_prefetch_mb << 20) / (2LL * pl->heads * vec_bytes)) : 0;
+      ranked && items >= 512 && pl->kv_prefetch_mb > 0 ? (int)(((long long)pl->kv_prefetch_mb << 20) / (2LL * pl->heads * vec_bytes)) : 0;
   auto prefetch = [&](const int32_t* sched, const void* k, const void* v, int cap) {
     KvPrefetch f{};
     if (prefetch_keys > 0 && k && v)

@@ -288,7 +288,7 @@ int b200dec_attention_q8(int self, const int32_t* active, const float* q, int ld
 int b200dec_row_schedule(const int32_t* active, const int32_t* pos, const int32_t* cross_len, int slots, int seq,
                          int frames, int rows, int prefetch_keys, int32_t* sched_self, int32_t* sched_cross,
                          int32_t* status, void* stream);
-/* b200dec_attention for a large batch (rows * heads >= 512 is where it pays), reading the rows from a schedule: the
+/* b200dec_attention for a large batch (rows * heads of 592 to 1036 is where it pays), reading the rows from a schedule: the
  * i-th longest row and the i-th shortest share a cluster of two CTAs that read the same number of keys; the partial
  * of the long row's tail crosses distributed shared memory. Same results as b200dec_attention up to the order of the
  * softmax merge. sched: (rows, 4) int32 from b200dec_row_schedule, 16-byte aligned. With pdl != 0 the kernel reads its
@@ -302,9 +302,10 @@ int b200dec_attention_paired(int self, const int32_t* sched, const float* q, int
 int b200dec_attention_paired_q8(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache,
                                 float* kscale, float* vscale, int heads, int head_dim, int cap, float scale, void* out,
                                 int out_kind, int rows, int pdl, void* stream);
-/* b200dec_attention for a middling batch (128 <= rows * heads < 512 is where it pays), reading the rows from a schedule as
- * b200dec_attention_paired does (the same rule for pdl): a cluster of up to four CTAs takes a (row, head), as many of them
- * as the row has 64 keys for share its keys. kscale, vscale: those of int8 caches, or both NULL for bf16 caches. */
+/* The same rows of a schedule (the same rule for pdl), longest first, each on a cluster of up to four CTAs: as many of them
+ * as the row has 64 keys for share its keys. With 4 x 148 items (rows * heads) or more the clusters are single CTAs. Pays
+ * from 128 items on, except where all rows are resident at once (592 to 1036), which is what b200dec_attention_paired is
+ * for. kscale, vscale: those of int8 caches, or both NULL for bf16 caches. */
 int b200dec_attention_spans(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache,
                             float* kscale, float* vscale, int heads, int head_dim, int cap, float scale, void* out,
                             int out_kind, int rows, int pdl, void* stream);
