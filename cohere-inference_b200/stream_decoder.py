@@ -243,6 +243,7 @@ class StreamDecoder:
             self.side_streams = [torch.cuda.Stream(device=dev, priority=-1) for _ in range(self.chains - 1)]
             self._build_plan()
             self._fused_ws = self._fused_workspaces(fused_rows)
+            self._fused_done = torch.cuda.Event()
             self._select_layers(min(self.buckets))
             self.launches_per_step = lib.b200dec_step_launches(C.byref(self.plan), min(self.buckets))
             self.weight_bytes = sum(p.stream_bytes() for ly in self.layers for p in ly.projections()) + \
@@ -430,20 +431,22 @@ class StreamDecoder:
         torch.cuda.current_stream().synchronize()
         return ws
 
-    # The CTAs of a fused step wait for one another, so two of them must not share the GPU: a decoder whose stream takes
-    # over from another decoder's waits for what that one has been given so far.
+    # The CTAs of a fused step wait for one another, so two of them must not share the GPU: a decoder's fused step waits
+    # for the newest one of any other decoder, through an event that every fused step leaves right behind itself. (Not one
+    # that the newcomer records on the other's stream: that stands behind everything the other decoder has been given
+    # since, its larger steps included, and the other's stream may be capturing in another thread.)
     _fused_lock = threading.Lock()
-    _fused_stream: dict[int, torch.cuda.Stream] = {}
+    _fused_last: dict[int, torch.cuda.Event] = {}  # by device
 
-    def _fused_turn(self) -> None:
-        """Call with the lock held, before a fused step is launched on the decoder stream."""
-        last = self._fused_stream.get(self.device.index)
-        if last is not self.stream:
-            if last is not None:
-                done = torch.cuda.Event()
-                done.record(last)
-                self.stream.wait_event(done)
-            self._fused_stream[self.device.index] = self.stream
+    def _in_turn(self, launch, bucket: int) -> None:
+        """launch(bucket), a fused step on the decoder stream, in its turn."""
+        with self._fused_lock:
+            last = self._fused_last.get(self.device.index)
+            if last is not None and last is not self._fused_done:
+                self.stream.wait_event(last)
+            launch(bucket)
+            self._fused_done.record(self.stream)
+            self._fused_last[self.device.index] = self._fused_done
 
     def _select_layers(self, b: int) -> None:
         """Points the plan at the layer packings bucket b runs on (a captured graph keeps what it was captured with)."""
@@ -501,9 +504,7 @@ class StreamDecoder:
         pool = torch.cuda.graph_pool_handle()
         with torch.cuda.device(self.device), torch.cuda.stream(self.stream):
             for rows in sorted(self.buckets, reverse=True):
-                with self._fused_lock:
-                    self._fused_turn()
-                    self._step(rows)
+                self._in_turn(self._step, rows)
                 self.stream.synchronize()
                 graph = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(graph, pool=pool, stream=self.stream):
@@ -657,9 +658,7 @@ class StreamDecoder:
         torch.cuda.nvtx.range_push("b200dec.step")
         with torch.cuda.stream(self.stream):
             if bucket in self._fused_ws:
-                with self._fused_lock:
-                    self._fused_turn()
-                    self._launch_step(bucket)
+                self._in_turn(self._launch_step, bucket)
             else:
                 self._launch_step(bucket)
         torch.cuda.nvtx.range_pop()
