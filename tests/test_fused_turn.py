@@ -97,6 +97,15 @@ def test_a_step_during_another_decoders_capture_stays_out_of_it(decoders):
     assert built.stream.waits and not any(s is built.stream and at > 3 for s, at in serving.stream.waits)
 
 
+def test_a_decoder_without_fused_steps_takes_no_turn(decoders):
+    serving, other = decoders((8,)), decoders(())
+    serving.step(8)
+    other._capture()
+    other.step(8)
+    serving.step(8)
+    assert not other.stream.waits and not serving.stream.waits
+
+
 def test_a_turn_is_waited_for_up_to_the_fused_step_only(decoders):
     """What the other decoder has been given besides (its steps of 128 rows) goes on beside this one's."""
     a, b = decoders((8,)), decoders((8,))
