@@ -660,11 +660,24 @@ class StreamDecoder:
         """One decoding step of `bucket` rows on the decoder stream (a graph replay)."""
         torch.cuda.nvtx.range_push("b200dec.step")
         with torch.cuda.stream(self.stream):
-            if bucket in self._fused_ws:
-                self._in_turn(self._launch_step, bucket)
-            else:
+            if bucket not in self._fused_ws:
                 self._launch_step(bucket)
+            elif not torch.cuda.is_current_stream_capturing():
+                self._in_turn(self._launch_step, bucket)
+            elif self.use_graphs:
+                self._launch_step(bucket)  # torch refuses to replay a graph inside a capture
+            else:
+                self._step_unfused(bucket)
         torch.cuda.nvtx.range_pop()
+
+    def _step_unfused(self, bucket: int) -> None:
+        """The step as the sequence of kernels, into a capture of the caller's: that graph is replayed without a turn."""
+        ws = self.plan.fused_ws
+        kept, ws[bucket - 1] = ws[bucket - 1], None
+        try:
+            self._step(bucket)
+        finally:
+            ws[bucket - 1] = kept
 
     def _launch_step(self, bucket: int) -> None:
         if self.use_graphs:

@@ -70,12 +70,12 @@ def decoders(monkeypatch):
         d.stream, d.device, d.buckets = _Stream(), SimpleNamespace(index=DEV), (8, 128)
         d._fused_ws, d.use_graphs, d.graphs = dict.fromkeys(fused), False, {}
         d._fused_done = _Event()
-        d.plan = SimpleNamespace(fused_ws=[None] * 16)
+        d.plan = SimpleNamespace(fused_ws=[b + 1 in fused or None for b in range(16)])
         d.reset = d.check_status = lambda: None
         d.during_capture = lambda: None
 
-        def step(b, *args, **kw):
-            d.stream.ops.append(b)
+        def step(b):
+            d.stream.ops.append(b if b > 16 or d.plan.fused_ws[b - 1] else (b, "kernel sequence"))
             if d.stream.capturing:
                 d.during_capture()
         d._step = step
@@ -118,6 +118,20 @@ def test_a_turn_is_waited_for_up_to_the_fused_step_only(decoders):
     assert len(b.stream.waits) == 1  # still its turn
     a.step(8)
     assert a.stream.waits == [(b.stream, 2)]
+
+
+def test_a_step_inside_a_callers_capture_takes_no_turn_and_is_not_fused(decoders):
+    """Nobody takes the turn when the caller's graph is replayed, so what it holds must not need one."""
+    a, b = decoders((8,)), decoders((8,))
+    a.step(8)
+    with torch.cuda.graph(None, stream=b.stream):
+        b.step(8)
+        b.step(8)
+    assert b.stream.ops == [(8, "kernel sequence")] * 2 and not b.stream.waits
+    a.step(8)
+    b.step(8)
+    assert a.stream.ops == [8, 8] and b.stream.ops[2:] == [8] and not a.stream.waits
+    assert b.stream.waits == [(a.stream, 2)]
 
 
 # ---- on the GPU -----------------------------------------------------------------------------------------------------
@@ -214,3 +228,33 @@ def test_a_fused_step_does_not_wait_for_another_decoders_larger_steps():
         b.step(small)
     assert np.array_equal(_tokens(b), _alone(1))
     a.check_status()
+
+
+@pytest.mark.gpu
+def test_a_replay_inside_a_callers_capture_stays_refused():
+    first, dec = _decoder(slots=8, buckets=(8,)), _decoder(slots=8, buckets=(8,))
+    first.step(_admit(first, 1))
+    b = _admit(dec, 0)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="during capturing stage"), torch.cuda.graph(torch.cuda.CUDAGraph(), stream=dec.stream):
+        dec.step(b)
+    for _ in range(55):
+        first.step(b)
+        dec.step(b)
+    assert np.array_equal(_tokens(dec), _alone(0))
+
+
+@pytest.mark.gpu
+def test_a_callers_capture_holds_the_kernel_sequence():
+    first, dec = _decoder(slots=8, buckets=(8,)), _decoder(slots=8, buckets=(8,), graphs=False)
+    first.step(_admit(first, 1))  # the newest turn is another decoder's
+    b = _admit(dec, 0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=dec.stream):
+        dec.step(b)
+    with torch.cuda.stream(dec.stream):
+        for i in range(55):
+            graph.replay() if i % 2 else dec.step(b)
+    # the two ways round differently, so tokens may part where two logits are as good as equal: the first ones may not
+    assert np.array_equal(_tokens(dec)[:, :16], _alone(0)[:, :16]) and int(dec.pos.sum()) == 8 * 55
