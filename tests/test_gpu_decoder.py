@@ -380,11 +380,13 @@ def _two_layers(heads):
 @pytest.mark.parametrize("kv_int8", [False, True])
 @pytest.mark.parametrize("rows", [1, 8, 9, 16])
 def test_fused_step_gives_what_the_kernel_sequence_gives(heads, mode, kv_int8, rows):
-    """Up to 16 rows a step runs as one cooperative kernel: the logits of the first and of later steps, the tokens and
+    """Up to 16 rows a step runs as one cooperative kernel: the logits of the first and of later steps, the choices and
     the positions are those of the kernel sequence. Row counts on both sides of the kernel's operand tiles (8, 16) and
     of one (row, head) per CTA (128 of them); contexts from the empty cache and one frame to more keys than one round
     of a warp's loads. Both sides stay within LOGIT_TOL of the oracle elsewhere; here they are held to it against one
-    another (fp16 operands, other summation orders)."""
+    another (fp16 operands, other summation orders), while the prompt is fed and both see the same tokens. Either side's
+    choice is the first maximum of its own logits, exactly; the two agree wherever the best logit leads by more than the
+    two errors; and past the prompt the choice is the token that is fed next."""
     model = _two_layers(heads)
     rng = np.random.default_rng(rows)
     frames = np.linspace(1, 300, rows).astype(int).tolist() if rows > 1 else [300]
@@ -395,10 +397,16 @@ def test_fused_step_gives_what_the_kernel_sequence_gives(heads, mode, kv_int8, r
         dec = _decoder(model, slots=rows, buckets=(rows,), max_new_tokens=8, max_prompt=150, max_audio_s=30.0, eos=-1,
                        record=True, kv_int8=kv_int8, fused_rows=fused_rows, **mode)
         assert dec.launches(rows) == 1 if fused_rows else dec.launches(rows) > 1
-        lg, _ = _run_teacher_forced(dec, memory, prompts, 150)
-        got.append((lg[[0, 1, 2, 40, 149]], dec.out.cpu().numpy()[:, :150], dec.pos.cpu().numpy()))
+        lg, am = _run_teacher_forced(dec, memory, prompts, 155)
+        out = dec.out.cpu().numpy()[:rows]
+        assert np.array_equal(am, lg.argmax(-1))
+        assert np.array_equal(out[:, 150:156], am[149:].T)
+        top = np.partition(lg[:150], -2, axis=-1)[..., -2:]
+        got.append((lg[[0, 1, 2, 40, 149]], out[:, :150], dec.pos.cpu().numpy(), am[:150], top[..., 1] - top[..., 0]))
     assert np.abs(got[0][0] - got[1][0]).max() <= LOGIT_TOL
     assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])
+    clear = got[0][4] > 2 * LOGIT_TOL
+    assert clear.mean() > 0.5 and np.array_equal(got[0][3][clear], got[1][3][clear])
 
 
 def test_fused_step_bounded_wait_runs_out_and_the_context_survives():
