@@ -647,12 +647,14 @@ def test_attention(nv, H, D, rows, self_, cap, ring):
 
 
 @pytest.mark.parametrize("H,D", [(16, 64), (8, 128)])
-@pytest.mark.parametrize("rows", [17, 24, 31])  # four, three and two CTAs per (row, head) of both head counts
+# CTAs per (row, head): with 16 heads 4, 3, 2, 2, 1, 1, 1, with 8 heads 4, 4, 4, 3, 2, 2, 1
+@pytest.mark.parametrize("rows", [10, 17, 24, 31, 40, 70, 128])
 @pytest.mark.parametrize("self_", [0, 1])
 @pytest.mark.parametrize("q8", [False, True])
 def test_attention_spans_against_one_cta_per_row(nv, H, D, rows, self_, q8):
     """A row's keys shared by a cluster: the same output as the kernel that gives every row one CTA, and the same bytes
-    appended. Lengths on both sides of every number of spans (64 keys each) and of the 16 keys a span is rounded to. bf16
+    appended; launched plainly and programmatically (behind a kernel that stands between it and the schedule's, as in the
+    step). Lengths on both sides of every number of spans (64 keys each) and of the 16 keys a span is rounded to. bf16
     caches: fp32 sums in another order. int8 caches: the weighted sums run through fp16 pairs whose chains a span
     shortens, half a unit (2^-11 of the largest value, |v| < 4) per addition of up to cap / 16 = 20 per lane."""
     cap = 320
@@ -673,12 +675,12 @@ def test_attention_spans_against_one_cta_per_row(nv, H, D, rows, self_, q8):
                                       cap, cap, rows, 0, nv.ptr(sched) if self_ else None,
                                       None if self_ else nv.ptr(sched), nv.ptr(status), nv.stream_ptr()))
     got = []
-    for spans in (False, True):
+    for pdl in (None, 0, 1):
         (k, v), (ks, vs) = [t.clone() for t in kv], [t.clone() if q8 else None for t in sc]
         out = torch.full((rows, H * D), 7.0, device="cuda")
-        if spans:
+        if pdl is not None:
             nv.check(lib.b200dec_attention_spans(self_, nv.ptr(sched), nv.ptr(q_d), ld, nv.ptr(k), nv.ptr(v), nv.ptr(ks),
-                                                 nv.ptr(vs), H, D, cap, scale, nv.ptr(out), nv.OUT_F32, rows, 0,
+                                                 nv.ptr(vs), H, D, cap, scale, nv.ptr(out), nv.OUT_F32, rows, pdl,
                                                  nv.stream_ptr()))
         elif q8:
             nv.check(lib.b200dec_attention_q8(self_, nv.ptr(a_d), nv.ptr(q_d), ld, nv.ptr(k), nv.ptr(v), nv.ptr(ks),
@@ -693,6 +695,8 @@ def test_attention_spans_against_one_cta_per_row(nv, H, D, rows, self_, q8):
     assert int(status.item()) == 0
     assert float((got[0][0] - got[1][0]).abs().max()) <= (20 * 4 * 2.0 ** -11 if q8 else 2e-5)
     for a, b in zip(got[0][1:], got[1][1:]):
+        assert torch.equal(a, b)
+    for a, b in zip(got[1], got[2]):
         assert torch.equal(a, b)
 
 
@@ -802,13 +806,14 @@ def test_scatter_kv_q8_bit_exact(nv, H, D):
 
 
 @pytest.mark.parametrize("H,D", [(16, 64), (8, 128)])
-@pytest.mark.parametrize("rows", [3, 41])   # one CTA per (row, head, split); rows paired in clusters
+# one CTA per (row, head, split); rows paired in clusters; spans of 4 CTAs, of 1 and 2 (16 and 8 heads), of 1
+@pytest.mark.parametrize("rows", [3, 41, 75])
 @pytest.mark.parametrize("self_", [0, 1])
-@pytest.mark.parametrize("paired", [False, True])
+@pytest.mark.parametrize("paired", [False, True, "spans"])
 def test_attention_q8(nv, H, D, rows, self_, paired):
     """Attention over int8 caches vs fp64 on the dequantised caches; the appended key and value are stored in the
     reference's int8 form (bit-exact) and attended in this step as their bf16 values."""
-    if paired and rows < 41:
+    if paired is True and rows < 41:
         pytest.skip("the schedule-driven kernel is for large batches")
     cap = 200
     rng = np.random.default_rng(rows + H + self_)
@@ -836,9 +841,9 @@ def test_attention_q8(nv, H, D, rows, self_, paired):
         nv.check(lib.b200dec_row_schedule(nv.ptr(a_d), nv.ptr(n_d) if self_ else None, None if self_ else nv.ptr(n_d), S,
                                           cap, cap, rows, 0, nv.ptr(sched) if self_ else None,
                                           None if self_ else nv.ptr(sched), nv.ptr(status), nv.stream_ptr()))
-        nv.check(lib.b200dec_attention_paired_q8(self_, nv.ptr(sched), nv.ptr(q_d), ld, nv.ptr(kd), nv.ptr(vd), nv.ptr(ksd),
-                                                 nv.ptr(vsd), H, D, cap, scale, nv.ptr(out), nv.OUT_F32, rows, 0,
-                                                 nv.stream_ptr()))
+        run = lib.b200dec_attention_spans if paired == "spans" else lib.b200dec_attention_paired_q8
+        nv.check(run(self_, nv.ptr(sched), nv.ptr(q_d), ld, nv.ptr(kd), nv.ptr(vd), nv.ptr(ksd), nv.ptr(vsd), H, D, cap, scale,
+                     nv.ptr(out), nv.OUT_F32, rows, 0, nv.stream_ptr()))
     else:
         nv.check(lib.b200dec_attention_q8(self_, nv.ptr(a_d), nv.ptr(q_d), ld, nv.ptr(kd), nv.ptr(vd), nv.ptr(ksd),
                                           nv.ptr(vsd), nv.ptr(n_d), S, H, D, cap, scale, nv.ptr(out), nv.OUT_F32, rows,
