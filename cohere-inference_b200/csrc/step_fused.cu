@@ -30,6 +30,15 @@ int fused_mode(const b200dec_plan* pl, int rows) {
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < FC)
     return -1;
+  // 16-bit weights at 9 to 16 rows: twice the weight pieces, a quarter of fc2 waiting in the ring, and every CTA polls the
+  // operand of all the rows (bf16 weights: as fp32). The sequence of kernels is ahead where its attention shares a row's
+  // keys, from 128 (row, head) items on (step.cu), and for bf16 weights a little earlier. Sequence / fused, us a step, ragged
+  // rows: 16 heads, fp16 248 / 261 at 9 rows, 268 / 292 at 16, bf16 284 / 292 and 309 / 350; 8 heads, fp16 309 / 290 at 15 rows,
+  // 280 / 298 at 16, bf16 355 / 343 at 14, 323 / 352 at 16; with all rows at 350 positions bf16 387 / 384 at 14, 385 / 394 at 15,
+  // over int8 caches 366 / 362 at 12, 365 / 376 at 13.
+  const int kind = pl->layer[0].qkv.kind, items = rows * pl->heads;
+  if (rows > 8 && ((kind == B200DEC_W_F16 && items >= 128) || (kind == B200DEC_W_BF16 && items >= (pl->kv_int8 ? 104 : 120))))
+    return -1;
   const bool a16 = pl->a_kind == B200DEC_A_F16;
   // a vocabulary projection in the fragment layout is taken with the operand precision its mode has here
   const bool head8 = h.kind == B200DEC_W_INT8_UMMA || (h.kind == B200DEC_W_INT8 && pl->head_a_kind == B200DEC_A_F16);

@@ -1172,8 +1172,11 @@ int launch_fused_mode(const FArgs& a, int head_dim, bool q8, cudaStream_t stream
   auto rows = [&](auto d, auto q) {
     constexpr int D = decltype(d)::value;
     constexpr bool Q = decltype(q)::value;
-    return a.rows > 8 ? go(fused_step_kernel<MODE, D, Q, true>, FTraits<MODE, true>::BYTES)
-                      : go(fused_step_kernel<MODE, D, Q, false>, FTraits<MODE, false>::BYTES);
+    if (a.rows <= 8) return go(fused_step_kernel<MODE, D, Q, false>, FTraits<MODE, false>::BYTES);
+    if constexpr (FTraits<MODE, true>::W16 && D == 64)  // 16 heads: 128 items and more, not fused (fused_mode)
+      return fail(B200DEC_EINVAL, "fused step: no kernel for %d rows of 16-bit weights and 16 heads", a.rows);
+    else
+      return go(fused_step_kernel<MODE, D, Q, true>, FTraits<MODE, true>::BYTES);
   };
   using i64 = std::integral_constant<int, 64>;
   using i128 = std::integral_constant<int, 128>;

@@ -397,7 +397,8 @@ int b200dec_compact_active(const b200dec_plan* plan, int rows, int32_t* n_active
 int b200dec_step(const b200dec_plan* plan, int rows, void* stream);
 /* 32-bit words of the workspace with which a step of `rows` rows runs as one kernel (plan->fused_ws[rows - 1]), or 0 when
  * this plan's steps of that size do not: more than 16 rows, weight kinds other than the mma.sync packings, the ring
- * attention kernel, a device of fewer than 128 SMs. */
+ * attention kernel, a device of fewer than 128 SMs, or more than 8 rows of 16-bit weights where the sequence of kernels is
+ * faster (from 128 (row, head) items on, bf16 weights from 120, over int8 caches from 104). */
 int64_t b200dec_fused_words(const b200dec_plan* plan, int rows);
 /* The same for rows [row0, row0 + rows) of the step's batch only. Disjoint row ranges share no scratch, so a caller
  * may run several ranges concurrently on forked streams to overlap one range's attention (bound by HBM) with another's
