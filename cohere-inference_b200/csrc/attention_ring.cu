@@ -320,8 +320,10 @@ __global__ void __launch_bounds__(NTHREADS, 2) attention_kernel(const AttnArgs p
           for (int r = 1; r < RND; ++r) nka[r] = nka[0], nkb[r] = nkb[0], nva[r] = nva[0], nvb[r] = nvb[0];
         }
       }
+      // the reads of the stage before the producer's next bulk copy into it: an arrival alone does not wait for them
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[st]);  // the stage's bytes are in registers
+      if (lane == 0) mbar_arrive(&empty[st]);
       if (append) {
         // The new key and value: rounded to bf16 into the cache at position n, and attended as stored, by the lanes
         // of key 0 of warp 0 (the other lanes and rounds go through `attend` masked: its shuffles need the whole warp).

@@ -321,8 +321,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) head_umma_kernel(const HeadArgs p
 #pragma unroll
       for (int j = 0; j < 2; ++j)
         r[j] = *reinterpret_cast<const uint4*>(raws + rs * RAW_BYTES + (2 * hf + j) * 2048 + ch * 16);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&raw_empty[rs]);  // the block's bytes are in registers
       ok = mbar_wait(&a_empty[st], ((kb / A_STAGES) & 1) ^ 1, p.wait_limit);
       if (!ok) break;
       unsigned char* row = as + st * A_BYTES + (ch >> 3) * 1024 + (ch & 7) * 128;
@@ -334,9 +332,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) head_umma_kernel(const HeadArgs p
         *reinterpret_cast<uint4*>(row + (((2 * pj) ^ (ch & 7)) << 4)) = lo;
         *reinterpret_cast<uint4*>(row + (((2 * pj + 1) ^ (ch & 7)) << 4)) = hi;
       }
-      fence_async_shared();
+      fence_async_shared();  // the tile to the MMAs, and the reads of the raw stage before its next bulk copy
       __syncwarp();
-      if (lane == 0) mbar_arrive(&a_full[st]);
+      if (lane == 0) mbar_arrive(&a_full[st]), mbar_arrive(&raw_empty[rs]);
     }
     if (!ok && lane == 0) atomicOr(p.status, B200DEC_ST_TIMEOUT);
 
@@ -606,8 +604,6 @@ __global__ void __launch_bounds__(HeadStream<UNS, W16>::NT, 1) head_stream_kerne
           if (ok) r[b] = *reinterpret_cast<const uint4*>(raws + rs * RAW_BYTES + pj * 2048 + ch * 16);
         }
         if (!ok) break;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&raw_empty[kb % RS]), mbar_arrive(&raw_empty[(kb + 1) % RS]);  // bytes are in registers
         // MMAs of blocks kb - AST and kb + 1 - AST are done: their weight and operand stages are free
 #pragma unroll
         for (int b = 0; b < 2; ++b)
@@ -624,9 +620,15 @@ __global__ void __launch_bounds__(HeadStream<UNS, W16>::NT, 1) head_stream_kerne
           *reinterpret_cast<uint4*>(row + (((2 * pj + 1) ^ (ch & 7)) << 4)) = hi;
         }
         cp_async_wait_group<LOOK>();  // this thread's pieces of operand blocks kb and kb + 1 (and earlier) have landed
+        // The fence stands for both hand-overs: the widened tile to the MMAs, and the raw stage back to the producer. An
+        // arrival right behind the reads would not do: it does not wait for them, and behind operand requests that the
+        // memory system is slow to take (another decoder on the GPU) they ran after the stage's next copy had landed.
         fence_async_shared();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&a_full[kb % AST]), mbar_arrive(&a_full[(kb + 1) % AST]);
+        if (lane == 0) {
+          mbar_arrive(&a_full[kb % AST]), mbar_arrive(&a_full[(kb + 1) % AST]);
+          mbar_arrive(&raw_empty[kb % RS]), mbar_arrive(&raw_empty[(kb + 1) % RS]);
+        }
       }
     }
     cp_async_wait_all();  // nothing of this thread's is on its way into the rings any more (also after a time-out)
