@@ -655,11 +655,12 @@ cudaError_t launch_spans(int head_dim, int self, dim3 grid, cudaStream_t s, int 
 
 }  // namespace
 
-extern "C" {
+namespace b200dec_detail {
 
-int b200dec_attention_spans(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache,
+// step_items: the (row, head) items of the whole step, of which these rows may be a part beside others (b200dec_step_part)
+int attention_spans_impl(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache,
                             float* kscale, float* vscale, int heads, int head_dim, int cap, float scale, void* out,
-                            int out_kind, int rows, int pdl, void* stream) {
+                            int out_kind, int rows, int64_t step_items, int pdl, void* stream) {
   B200_REQUIRE(sched && q && kcache && vcache && out, "attention_spans: null pointer");
   B200_REQUIRE((kscale == nullptr) == (vscale == nullptr), "attention_spans: key and value scales go together");
   B200_REQUIRE(head_dim == 64 || head_dim == 128, "attention_spans: head_dim %d (64 or 128)", head_dim);
@@ -672,13 +673,23 @@ int b200dec_attention_spans(int self, const int32_t* sched, const float* q, int 
   p.q = q, p.k = (__nv_bfloat16*)kcache, p.v = (__nv_bfloat16*)vcache, p.ks = kscale, p.vs = vscale;
   p.sched = sched, p.out = out, p.ldq = ldq, p.H = heads, p.cap = cap, p.out_kind = out_kind, p.rows = rows;
   p.scale_log2 = scale * 1.4426950408889634f;
-  const int64_t items = (int64_t)rows * heads;
-  const int want = (int)((4 * 148 + items - 1) / items);  // four CTAs per SM
+  const int want = (int)((4 * 148 + step_items - 1) / step_items);  // four CTAs per SM
   const dim3 grid(want < SPAN_MAX ? want : SPAN_MAX, heads, rows);
   const cudaError_t e = kscale ? launch_spans<true>(head_dim, self, grid, (cudaStream_t)stream, pdl, p)
                                : launch_spans<false>(head_dim, self, grid, (cudaStream_t)stream, pdl, p);
   if (e != cudaSuccess) return fail(B200DEC_ECUDA, "attention_spans launch: %s", cudaGetErrorString(e));
   return 0;
+}
+
+}  // namespace b200dec_detail
+
+extern "C" {
+
+int b200dec_attention_spans(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache,
+                            float* kscale, float* vscale, int heads, int head_dim, int cap, float scale, void* out,
+                            int out_kind, int rows, int pdl, void* stream) {
+  return attention_spans_impl(self, sched, q, ldq, kcache, vcache, kscale, vscale, heads, head_dim, cap, scale, out, out_kind,
+                              rows, (int64_t)rows * heads, pdl, stream);
 }
 
 int64_t b200dec_attention_scratch_floats(int rows, int heads, int head_dim) {

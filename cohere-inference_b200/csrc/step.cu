@@ -24,6 +24,9 @@ int pick_impl(const float* part_max, const int32_t* part_idx, int partials, cons
               int64_t* tok, int32_t* pos, uint8_t* finished, const int64_t* forced, int max_prompt,
               const int32_t* plen, const int32_t* limit, int64_t* out, int out_cols, int eos, int64_t* argmax,
               uint8_t* flags_host, int pdl, void* stream);
+int attention_spans_impl(int self, const int32_t* sched, const float* q, int ldq, void* kcache, void* vcache, float* kscale,
+                         float* vscale, int heads, int head_dim, int cap, float scale, void* out, int out_kind, int rows,
+                         int64_t step_items, int pdl, void* stream);
 bool fused_step_applies(const b200dec_plan* pl, int row0, int rows);
 int fused_step(const b200dec_plan* pl, int rows, void* stream);
 }  // namespace b200dec_detail
@@ -72,11 +75,13 @@ int b200dec_step_launches(const b200dec_plan* pl, int rows) {
   return n;
 }
 
-// Rows [row0, row0 + rows) of the step's batch as one chain of kernels. Every scratch buffer is indexed by row, so
+// Rows [row0, row0 + rows) of a step of step_rows rows (0: not known) as one chain of kernels. Every scratch buffer is indexed by row, so
 // disjoint row ranges may run concurrently on different streams (the caller forks and joins them).
-int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) {
+int b200dec_step_part(const b200dec_plan* pl, int row0, int rows, int step_rows, void* stream) {
   B200_REQUIRE(pl && pl->layer && pl->layers >= 1, "step: null plan or no layers");
   B200_REQUIRE(rows >= 1 && row0 >= 0 && row0 + rows <= 128, "step: rows %d + %d outside 0..128", row0, rows);
+  B200_REQUIRE(step_rows == 0 || (step_rows >= row0 + rows && step_rows <= 128), "step: rows %d + %d of a step of %d", row0,
+               rows, step_rows);
   B200_REQUIRE(pl->heads * pl->head_dim == D_MODEL, "step: heads * head_dim must be %d", D_MODEL);
   B200_REQUIRE(pl->vocab == pl->head.n, "step: vocab %d vs head rows %d", pl->vocab, pl->head.n);
   B200_REQUIRE(!(pl->kv_int8 && pl->attn_ring), "step: the ring attention kernel reads bf16 caches only");
@@ -148,9 +153,15 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
   // resident and the longest decides, long rows are paired with short ones. Paired / this way, us a step, ragged rows at
   // position 30-270: 512 items 477 / 443 (8 x 128, fp16), 371 / 341 (16 x 64, int8 caches); 1536 585 / 543, 559 / 504 and
   // 2048 669 / 635, 623 / 574 (16 x 64, bf16 / int8 caches); paired the better one at 768 (620 / 666) and 896 (678 / 723).
-  const int items = rows * pl->heads;
+  // With rows of one length there is less between the two: 1536 558 / 551 and 512 / 511, 2048 644 / 636 and 578 / 577.
+  // A part of a step runs beside the other parts, whose CTAs fill the SMs too: it is never paired, and how many CTAs share a
+  // row follows from the items of the whole step. By the part's own items / by the step's, us a step, short, ragged and long
+  // contexts: 2 x 32 rows, 16 x 64, 439 / 398, 520 / 488, 624 / 579 (paired 408, 499, 586); 4 x 16 rows, 8 x 128, int8
+  // caches, 574 / 535, 658 / 590, 729 / 647. Where the whole is not known (step_rows 0): as if alone, but paired from 512 items.
+  const int items = rows * pl->heads, step_items = step_rows ? step_rows * pl->heads : items;
   const bool ranked = !pl->attn_ring && pl->sched_self && pl->sched_cross && items >= 128 && rows <= 256;
-  const bool paired = ranked && items >= 4 * 148 && items <= 7 * 148, spans = ranked && !paired;
+  const bool paired = ranked && items == step_items && items >= (step_rows ? 4 * 148 : 512) && items <= 7 * 148;
+  const bool spans = ranked && !paired;
   int32_t* sched_self = ranked ? pl->sched_self + 4 * row0 : nullptr;
   int32_t* sched_cross = ranked ? pl->sched_cross + 4 * row0 : nullptr;
 
@@ -191,9 +202,10 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
     // a pair could see different versions of an entry and disagree on their hand-off: it is then launched plainly.
     const int pdl_self = (i == 0 && !(want & 2)) ? 0 : pdl_attn;
     if (spans)
-      B200_TRY_IN(4, b200dec_attention_spans(1, sched_self, qkv, 3 * hd, ly.self_k, ly.self_v,
+      B200_TRY_IN(4, attention_spans_impl(1, sched_self, qkv, 3 * hd, ly.self_k, ly.self_v,
                                              pl->kv_int8 ? ly.self_ks : nullptr, pl->kv_int8 ? ly.self_vs : nullptr,
-                                             pl->heads, pl->head_dim, pl->seq, scale, att, ok_a, rows, pdl_self, stream));
+                                             pl->heads, pl->head_dim, pl->seq, scale, att, ok_a, rows, step_items,
+                                          pdl_self, stream));
     else if (pl->kv_int8 && paired)
       B200_TRY_IN(4, b200dec_attention_paired_q8(1, sched_self, qkv, 3 * hd, ly.self_k, ly.self_v, ly.self_ks, ly.self_vs,
                                            pl->heads, pl->head_dim, pl->seq, scale, att, ok_a, rows, pdl_self, stream));
@@ -213,9 +225,10 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
     B200_TRY_IN(2, linear_impl(&ly.cq, ln_src, ln_kind, &ly.ln2, D_MODEL, rows, cq, B200DEC_OUT_F32, hd, B200DEC_ACT_NONE, pdl,
                          stream, &r2, nullptr));
     if (spans)
-      B200_TRY_IN(4, b200dec_attention_spans(0, sched_cross, cq, hd, (void*)ly.cross_k, (void*)ly.cross_v,
+      B200_TRY_IN(4, attention_spans_impl(0, sched_cross, cq, hd, (void*)ly.cross_k, (void*)ly.cross_v,
                                              pl->kv_int8 ? ly.cross_ks : nullptr, pl->kv_int8 ? ly.cross_vs : nullptr,
-                                             pl->heads, pl->head_dim, pl->frames, scale, att, ok_a, rows, pdl_attn, stream));
+                                             pl->heads, pl->head_dim, pl->frames, scale, att, ok_a, rows,
+                                          step_items, pdl_attn, stream));
     else if (pl->kv_int8 && paired)
       B200_TRY_IN(4, b200dec_attention_paired_q8(0, sched_cross, cq, hd, (void*)ly.cross_k, (void*)ly.cross_v, ly.cross_ks,
                                            ly.cross_vs, pl->heads, pl->head_dim, pl->frames, scale, att, ok_a, rows,
@@ -252,6 +265,10 @@ int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) 
   return 0;
 }
 
-int b200dec_step(const b200dec_plan* pl, int rows, void* stream) { return b200dec_step_rows(pl, 0, rows, stream); }
+int b200dec_step_rows(const b200dec_plan* pl, int row0, int rows, void* stream) {
+  return b200dec_step_part(pl, row0, rows, 0, stream);
+}
+
+int b200dec_step(const b200dec_plan* pl, int rows, void* stream) { return b200dec_step_part(pl, 0, rows, rows, stream); }
 
 }  // extern "C"

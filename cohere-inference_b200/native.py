@@ -127,6 +127,7 @@ PROTOTYPES = {
     "b200dec_step": (C.c_int, [C.POINTER(Plan), C.c_int, vp]),
     "b200dec_fused_words": (i64, [C.POINTER(Plan), C.c_int]),
     "b200dec_step_rows": (C.c_int, [C.POINTER(Plan), C.c_int, C.c_int, vp]),
+    "b200dec_step_part": (C.c_int, [C.POINTER(Plan), C.c_int, C.c_int, C.c_int, vp]),
     "b200dec_step_launches": (C.c_int, [C.POINTER(Plan), C.c_int]),
 }
 

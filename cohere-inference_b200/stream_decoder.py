@@ -470,7 +470,7 @@ class StreamDecoder:
             for (r0, n), side in zip(ranges, [main] + self.side_streams):
                 if side is not main:
                     side.wait_event(fork)
-                nv.check(nv.lib().b200dec_step_rows(C.byref(self.plan), r0, n, side.cuda_stream))
+                nv.check(nv.lib().b200dec_step_part(C.byref(self.plan), r0, n, b, side.cuda_stream))
                 if side is not main:
                     done = torch.cuda.Event()
                     done.record(side)

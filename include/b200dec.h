@@ -404,6 +404,9 @@ int64_t b200dec_fused_words(const b200dec_plan* plan, int rows);
  * may run several ranges concurrently on forked streams to overlap one range's attention (bound by HBM) with another's
  * projections (bound by latency). No counterpart in the reference, which runs the batch as one chain. */
 int b200dec_step_rows(const b200dec_plan* plan, int row0, int rows, void* stream);
+/* The same with the rows of the whole step (0: not known, which is b200dec_step_rows): ranges that run side by side share
+ * the SMs, and the attention divides its rows among as many CTAs as that leaves room for. */
+int b200dec_step_part(const b200dec_plan* plan, int row0, int rows, int step_rows, void* stream);
 /* Kernels b200dec_step launches for `rows` rows (for launch accounting). */
 int b200dec_step_launches(const b200dec_plan* plan, int rows);
 

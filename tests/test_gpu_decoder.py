@@ -3,6 +3,7 @@ seeded weights and inputs. Tolerances are the ones the benchmark definition stat
 max-abs of the fp32 path on the weights the mode stores (dequantised int8 / bf16-rounded), greedy agreement >= 99.5 %
 under teacher forcing."""
 
+import ctypes
 import functools
 import os
 
@@ -410,6 +411,35 @@ def test_fused_step_gives_what_the_kernel_sequence_gives(heads, mode, kv_int8, r
     assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])
     clear = got[0][4] > 2 * LOGIT_TOL
     assert clear.mean() > 0.5 and np.array_equal(got[0][3][clear], got[1][3][clear])
+
+
+@pytest.mark.parametrize("rows,chains", [(32, 4), (64, 2), (72, 3), (128, 3)])
+@pytest.mark.parametrize("heads,kv_int8", [(16, False), (8, True)])
+def test_chains_give_what_one_chain_gives(heads, kv_int8, rows, chains):
+    """A step's rows as several chains that run side by side: the logits of one chain. Parts below and above 128 and 512
+    (row, head) items, of one and of unequal sizes; a row's keys go to three CTAs, two or one, by the items of the whole
+    step. The rows as unrelated calls of b200dec_step_rows give them too; a part that is none is refused."""
+    from cohere_inference_b200 import native as nv
+    model = _two_layers(heads)
+    rng = np.random.default_rng(rows)
+    frames = rng.permutation(np.linspace(1, 375, rows).astype(int)).tolist()
+    memory = [rng.standard_normal((t, 1024)).astype(np.float32) for t in frames]
+    prompts = [rng.integers(0, 16384, 24).astype(np.int64) for _ in range(rows)]
+    got = []
+    for c, part in ((1, None), (chains, None), (chains, nv.lib().b200dec_step_rows)):
+        dec = _decoder(model, slots=rows, buckets=(rows,), max_new_tokens=8, max_prompt=24, max_audio_s=30.0, eos=-1,
+                       record=True, kv_int8=kv_int8, int8=True, chains=c, graphs=False)
+        if part:
+            def step(b, dec=dec):
+                for r0, n in dec.row_ranges(b):
+                    nv.check(part(ctypes.byref(dec.plan), r0, n, dec.stream.cuda_stream))
+            dec._step = step
+        lg, _ = _run_teacher_forced(dec, memory, prompts, 24)
+        got.append(lg[[0, 1, 11, 23]])
+    assert all(np.abs(g - got[0]).max() <= LOGIT_TOL for g in got[1:])
+    for r0, n, whole in ((0, rows, rows - 1), (8, rows - 8, rows - 8), (0, 8, 129), (0, 8, -1)):
+        with pytest.raises(nv.NativeError, match="of a step of"):
+            nv.check(nv.lib().b200dec_step_part(ctypes.byref(dec.plan), r0, n, whole, dec.stream.cuda_stream))
 
 
 def test_fused_step_bounded_wait_runs_out_and_the_context_survives():
