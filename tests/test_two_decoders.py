@@ -75,3 +75,46 @@ def test_a_decoder_beside_another_gives_the_bits_it_gives_alone(first, second):
             t.join()
         for i in range(2):
             assert np.array_equal(got[i], alone[i]), (i, np.argwhere(got[i] != alone[i])[:8])
+
+
+@pytest.mark.parametrize("rows,kw", [(8, dict(int8=True)), (24, dict(int8=True)), (64, dict(int8=True, kv_int8=True)),
+                                     (24, dict(fp16_weights=True)), (8, dict())])
+def test_steps_and_prefills_side_by_side_give_their_bits(rows, kw):
+    """Clips that are admitted while others decode: their prefill runs on a stream of its own beside the steps in flight,
+    as DecodeScheduler has it."""
+    from cohere_inference_b200 import StreamDecoder
+    dec = StreamDecoder(_model(), slots=rows + 8, buckets=(rows,), max_new_tokens=8, max_prompt=STEPS, max_audio_s=30.0,
+                        eos=-1, record=True, **kw)
+    names = ["cross_k", "cross_v"] + (["cross_ks", "cross_vs"] if kw.get("kv_int8") else [])
+    lens, slots = [375, 300, 77, 1, 129, 250, 375, 33], list(range(rows, rows + 8))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    clips = [torch.randn(sum(lens), 1024, device="cuda", generator=g).to(t) for t in (torch.float32, torch.bfloat16)]
+
+    def caches():
+        return [torch.cat([getattr(dec, n)[:, s, :, :f].flatten() for s, f in zip(slots, lens)]) for n in names]
+    want = []
+    for x in clips:
+        with torch.cuda.stream(dec.stream):
+            dec.stream.wait_stream(torch.cuda.default_stream())
+            dec.fill_cross(x, lens, slots)
+        dec.check_status()
+        want.append(caches())
+    alone = _steps(dec, rows, _admit(dec, rows, 0))
+    bucket, got, stop, fills = _admit(dec, rows, 0), [], threading.Event(), [0]
+
+    def serve():
+        got.append(_steps(dec, rows, bucket))
+        stop.set()
+    t = threading.Thread(target=serve)
+    side = torch.cuda.Stream()
+    t.start()
+    while not stop.is_set() or fills[0] < 2:
+        i = fills[0] % 2
+        with torch.cuda.stream(side):
+            dec.fill_cross(clips[i], lens, slots)
+            now = caches()
+        side.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(now, want[i]))
+        fills[0] += 1
+    t.join()
+    assert np.array_equal(got[0], alone)
