@@ -8,10 +8,11 @@
 //     operands are stored in global memory as the exact shared-memory image of their tiles (K-major rows of 128 bytes
 //     with the 128-byte swizzle, 16 KB per 128-row block of a half of A, 32 KB per 256-channel block of B), so a pipeline
 //     stage is three plain cp.async.bulk copies that complete on an mbarrier; nothing else touches the operands. A stage
-//     holds 64 k of both halves and of the weights, so that the weights enter shared memory once: the multiply of a
-//     stage takes 1024 cycles, its 64 KB at 64 bytes a cycle from L2 as long. (As one product over 2 K with the weights
-//     fetched for either half it was 96 KB, and bound by them: 64 clips, 13 600 frames, 906 -> 819 us a
-//     prefill, 1.07 -> 1.18 PFLOP/s of the two halves.)
+//     holds 64 k of both halves and of the weights, so that the weights enter shared memory once: 64 KB against 1024 cycles
+//     of multiply, where one product over 2 K that fetches the weights for either half copies 96 KB. 64 clips, 13 600 frames,
+//     call after call: 850 -> 761 us, 1.14 -> 1.28 PFLOP/s of the two halves, which is where the power cap holds a long GEMM on
+//     this chip (cuBLAS 1.39); a single call on a cool chip 743 -> 663 us, 1.30 -> 1.46 (13 534 frames). The tensor pipe is
+//     active for 80 % of the second product's cycles (73 % before), the rest is the head and the tail of the tile lists.
 //   * persistent CTAs, one per SM, walk the (n tile, m tile) list; warp 0 feeds a 3-stage ring, warp 1 issues
 //     tcgen05.mma (M 128, N 256, K 16; 8 per stage) into one of two 256-column accumulators in tensor memory and
 //     commits stage releases and tile completion to mbarriers, warps 2-5 drain the other accumulator with tcgen05.ld

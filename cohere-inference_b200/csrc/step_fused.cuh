@@ -21,9 +21,12 @@
 //   * Attention: one CTA per (row, head) of up to 128, two per CTA above that; caches are asked into L2 a stage early and
 //     the first keys are in registers before the query arrives. (Splitting the keys of 1-2 rows over idle CTAs made every
 //     CTA poll 16 KB of partial outputs instead of 2 KB and cost more than it gave.)
-// With all that the step is bound by the exchanges (about 1.3 us from a result to its arrival in every CTA's registers,
-// most of it L2: the same few lines go to 128 SMs) and by the instructions between two of them (four warps per
-// scheduler, each a dependent chain), so the code is kept short in both senses. The loop over the layers runs through ONE
+// Where the time goes, from clock stamps (1 row, 16 x 64 heads, bf16 caches, 175 frames, 152 us): the 64 stages take 119 us,
+// 0.4-0.8 us each from the last barrier to the first poll (sums, epilogue, publishing, the next stage's prologue), 0.15 in
+// the hold below, 0.4-0.6 polling (the same few lines go to 128 SMs through L2), 0.1-0.7 multiplying or attending; the
+// vocabulary projection 9.7; the rest is the launch, the embedding, the first layer's copies and the pick. So the code is kept
+// short between two exchanges and in itself. 8 x 128 heads over int8 caches take 196 us: the two attention stages of a layer
+// wait 2.2 us each in front of the first keys, whose scales nobody has asked into L2 (bf16 caches: 0.6). The loop over the layers runs through ONE
 // copy each of the LayerNorm-folding projection, the output projection, fc2 and the attention, driven by a table in
 // shared memory: with a copy per stage it was 120 KB of instructions that every layer fetched again (265 us at 1 row).
 // And each copy does only what its kind needs: one general projection for all six executed 935 instructions per warp
@@ -257,8 +260,13 @@ struct FusedStep {
   }
   // Nothing another CTA publishes can be here before it has had the time of a trip through L2 since this CTA's own last
   // result, and looking earlier costs the others: polls of lines that every CTA reads queue up in front of the stores to
-  // them. (8 rows: 246 us a step without the hold, 183 with it.)
-  static constexpr uint32_t HOP = 1400, IDLE = 1500;  // cycles; IDLE: more where the CTA has had no (row, head) to attend
+  // them. A trip through L2 is what it is on this chip at its full clock: us a step with a hold of 0 / 700 / 1400 / 2100
+  // cycles, 16 x 64 heads and bf16 caches, 1 row 194 / 163 / 152 / 168, 8 rows 258 / 218 / 186 / 188, 16 rows 236 / 238 / 240 /
+  // 239 (there the polls are slower than the hold); 8 x 128 heads over int8 caches 240 / 207 / 196 / 211, 290 / 251 / 215 / 225,
+  // 250 / 250 / 252 / 249.
+  // IDLE: more where the CTA has had no (row, head) to attend. 0, 1500 and 3000 cycles are the same within 0.3 us except at
+  // 16 rows over int8 caches (252.7, 251.6, 252.0).
+  static constexpr uint32_t HOP = 1400, IDLE = 1500;  // cycles
   uint32_t since = 0;      // clock at the last barrier
   DEVI static uint32_t now() {
     uint32_t c;
